@@ -197,16 +197,18 @@ static int run_reverse(tc_ctx *ctx, int wavelet, int rounding, const void *const
     return TC_OK;
 }
 
-void t1_class_order(const tc_cblk_desc *h_desc, int n, uint32_t *h_order, int counts[6])
+void t1_class_order(const tc_cblk_desc *h_desc, int n, uint32_t *h_order, int counts[6], int planes[2])
 {
     std::vector<uint32_t> all(n);
     tc_t1_sort_order(h_desc, n, all.data());
     std::vector<uint32_t> cls[6];
+    planes[0] = planes[1] = 0;
     for (uint32_t i : all) {
         const tc_cblk_desc &d = h_desc[i];
         const int nb = d.passes ? (int)d.mb - (int)d.zero_bitplanes : 0;
         const int k = (nb <= 8 ? 0 : (nb <= 16 ? 1 : 2)) + ((d.style & kStyleDecodeBits) ? 3 : 0);
         cls[k].push_back(i);
+        planes[k / 3] = std::max(planes[k / 3], std::min(nb, 31));
     }
     int o = 0;
     for (int k = 0; k < 6; k++) {
@@ -260,6 +262,7 @@ struct tc_plan {
     const void *preloaded = nullptr;
     uint64_t preloaded_len = 0;
     int class_counts[6] = {0, 0, 0, 0, 0, 0};  // Tier-1 blocks of <= 8, <= 16, <= 31 coded bit-planes; styled ones alike
+    int t1_planes[2] = {0, 0};                 // most coded bit-planes of a plain and of a styled block
     bool profiling = false;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     PinBuf h_pool, h_desc, h_order;  // pinned host staging, alive until the next build
@@ -369,7 +372,7 @@ static int plan_build_parsed(tc_ctx *ctx, const Parsed *const *parsed, const uin
         }
         po += (pl + 15) & ~uint64_t(15);
     }
-    t1_class_order(hdesc, P->ncblk, horder, P->class_counts);
+    t1_class_order(hdesc, P->ncblk, horder, P->class_counts, P->t1_planes);
     P->pool_len = pool_total;
     P->scratch_per_img = scratch_max;
     cudaStream_t st = ctx->stream;
@@ -629,7 +632,7 @@ static int plan_run(tc_plan *P, void *const *d_out, bool graph_mode = false)
                                       P->class_counts[1], P->class_counts[2],
                                       static_cast<uint8_t *>(P->pool.ptr), graph_mode ? P->pool.size : P->pool_len,
                                       P->coef.ptr, P->coef.size / 4, TC_T1_OUT_DEQUANT, P->recon_r,
-                                      P->class_counts + 3);
+                                      P->class_counts + 3, P->t1_planes);
     if (e != cudaSuccess) return cuda_status(ctx, e, "Tier-1 launch");
     if (P->profiling) cudaEventRecord(P->ev[1], ctx->stream);
     if (graph_mode || plan_batched(P)) {
@@ -1164,10 +1167,10 @@ static void plan_graph_key(const tc_plan *P, void *const *d_out, std::vector<uin
     const int *cc = P->class_counts;
     topo = {(uint64_t)P->ctx->t1_group, (uint64_t)P->dwt_launches.size()};
     for (int k = 0; k < 6; k++) topo.push_back(cc[k] > 0);
-    // the heavy queue and the 8-in-16 merge change the Tier-1 launches
-    topo.push_back(cc[0] > 0 && cc[1] > 0 && cc[1] <= 148 && 8 * cc[1] <= cc[0]);
+    // the choice of kernel and the 8-in-16 merge of lane groups change the
+    // Tier-1 launches
+    topo.push_back(t1_warp_deep(P->ctx, cc[0] + cc[1] + cc[2]));
     topo.push_back(cc[0] > 0 && cc[1] > 0 && 2 * cc[0] <= cc[1]);
-    topo.push_back(cc[3] > 0 && cc[4] > 0 && cc[4] <= 148 && 8 * cc[4] <= cc[3]);
     for (const tc_plan::DwtLaunch &L : P->dwt_launches)
         for (int v : {L.wavelet, L.color, L.ncomp, L.otype, L.bits}) topo.push_back((uint64_t)(int64_t)v);
     key = topo;
@@ -1179,6 +1182,7 @@ static void plan_graph_key(const tc_plan *P, void *const *d_out, std::vector<uin
                        (uint64_t)(uintptr_t)P->jobs.ptr, (uint64_t)rbits})
         key.push_back(v);
     for (int k = 0; k < 6; k++) key.push_back((uint64_t)cc[k]);
+    for (int k = 0; k < 2; k++) key.push_back((uint64_t)P->t1_planes[k]);
     for (const tc_plan::DwtLaunch &L : P->dwt_launches)
         for (int v : {L.first, L.njobs, L.ntiles}) key.push_back((uint64_t)v);
     // images without a transform take their colour launch's pointers as

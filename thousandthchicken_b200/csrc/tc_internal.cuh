@@ -159,20 +159,32 @@ int cuda_status(tc_ctx *ctx, cudaError_t e, const char *what);
 // ---- kernels' host launchers (each returns a cudaError_t of the launch) ----
 
 // One persistent launch over n blocks whose coded bit-planes are at most
-// max_bitplanes (selects the magnitude storage width: 8, 16 or 32 bits).
+// max_bitplanes (rounded up to 8, 16 or 31: a block above that is flagged).
 cudaError_t launch_t1_decode(tc_ctx *ctx, const tc_cblk_desc *d_desc, const uint32_t *d_order,
                              int n, const uint8_t *d_pool, uint64_t pool_len, void *d_out,
                              uint64_t out_elems, int out_mode, float recon_r, int max_bitplanes);
 // Persistent launches over an order array partitioned into blocks of at
 // most 8, 16 and 31 coded bit-planes (n8 + n16 + n32 entries), then blocks
 // with a code-block style in the same three widths (nstyled[0..2], or none).
+// planes: the most coded bit-planes of a plain and of a styled block, when
+// the caller knows them (the decoder's state is sized for them).
 cudaError_t launch_t1_classes(tc_ctx *ctx, const tc_cblk_desc *d_desc, const uint32_t *d_order,
                               int ndesc, int n8, int n16, int n32, const uint8_t *d_pool,
                               uint64_t pool_len, void *d_out, uint64_t out_elems, int out_mode,
-                              float recon_r, const int *nstyled = nullptr);
+                              float recon_r, const int *nstyled = nullptr, const int *planes = nullptr);
+// One launch of the one-warp-per-block decoder over up to three slices of
+// blocks, taken in turn; max_planes: the most coded bit-planes of a block (one
+// above it is flagged); word: the work counter in d_words.
+cudaError_t launch_t1_warp(tc_ctx *ctx, bool styled, const tc_cblk_desc *d_desc, const uint32_t *const order[3],
+                           const int n[3], int ndesc, int max_planes,
+                           const uint8_t *d_pool, uint64_t pool_len, void *d_out, uint64_t out_elems, int out_mode,
+                           float recon_r, int word);
+// Whether it decodes n plain blocks with its kernel for few blocks.
+bool t1_warp_deep(const tc_ctx *ctx, int n);
 // Host: order longest-first within each class (<= 8, <= 16, <= 31 coded
-// bit-planes, then styled blocks of <= 8, <= 16, <= 31); class sizes out.
-void t1_class_order(const tc_cblk_desc *h_desc, int n, uint32_t *h_order, int counts[6]);
+// bit-planes, then styled blocks of <= 8, <= 16, <= 31); class sizes and the
+// most bit-planes of a plain and of a styled block out.
+void t1_class_order(const tc_cblk_desc *h_desc, int n, uint32_t *h_order, int counts[6], int planes[2]);
 cudaError_t launch_dequant_raw(tc_ctx *ctx, const tc_cblk_desc *d_desc, int n,
                                const uint32_t *d_raw, void *d_out, uint64_t elems, float recon_r);
 cudaError_t launch_t1_encode(tc_ctx *ctx, const tc_t1_enc_desc *d_desc, int n, const void *d_in, uint8_t *d_out,
