@@ -6,16 +6,25 @@
 // (t1_encode_block in j2k_host.cpp): all coding passes, or the first
 // max_passes of them, MQ termination by the FLUSH procedure of ISO C.2.9.
 //
-//   * one warp per code-block, CTAs of kEncWarps blocks; at every bit-plane
-//     the lanes rebuild the plane's bits per column from the input (float
-//     quantised with the band's step, or int32), read coalesced and cached,
-//     so a block's state is 5.7 KB of shared memory;
-//   * the coding state is the decoder's flag-word layout (t1_common.cuh):
-//     at every stripe the lanes find the candidate columns of the pass with
-//     __ballot_sync and the serial loop visits only those, in scan order;
-//   * the MQ encoder (ISO C.2) keeps A, C, CT and the last output byte in
-//     registers, replicated across the lanes; lane 0 writes the bytes once
-//     they can no longer take a carry.
+// One warp per code-block.  The samples are known, so only the MQ coder is
+// serial: for every stripe of a pass the lanes work out in parallel which
+// samples the pass codes, their contexts and signs, and put the decisions
+// (context label, bit) into a list in scan order; the warp then runs the list
+// through the MQ coder in lock-step.
+//   * a lane holds two columns of the block (c and c + 32) as 64-bit masks in
+//     registers: significance, signs, the plane's bits, visited, refined; its
+//     neighbours' rows come by shuffles;
+//   * in the significance propagation pass a sample that becomes significant
+//     makes its later neighbours candidates: the lanes iterate this to its
+//     fixed point, columns to the left first seen as they will be by then;
+//   * a sample's context sees the column to the left and the row above it as
+//     this pass leaves them, the rest as it found them.
+// The coder is bound by the decisions' chain when blocks are few and by issue
+// slots when they fill the GPU; the list takes the context search that ran
+// between decisions off both (64x64 blocks of 9 bit-planes: 48 of them 8.4 ->
+// 3.45 ms, 3,072 11.8 -> 7.6 ms, 12,288 42.2 -> 23.5 ms).  80 registers, six
+// CTAs (24 warps) per SM: at 96 and five, 768 CTAs left a second wave of 28
+// (8.1 ms); at 64 registers every block took 37% longer.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -26,19 +35,50 @@
 namespace tc {
 namespace {
 
-constexpr int kEncWarps = 8;
+constexpr int kEncWarps = 4;   // code-blocks per CTA
+constexpr int kSymRun = 72, kSymUni = 68;   // labels are kept as byte offsets (4 x label)
 
-// A block's coding state: 5.7 KB, so that 32 warps fit an SM.  The
-// magnitudes are not kept: at every bit-plane the lanes rebuild that
-// plane's bits per column from the (cached) input.
-struct EncState {
-    uint32_t F[kMaxStripes * 64];       // flag word per stripe column
-    unsigned long long sgn[kSgnCols];   // sign of the significant samples per column
-    unsigned long long neg[64];         // sign of every sample per column (bit y)
-    unsigned long long bits[64];        // the current bit-plane per column (bit y)
-    uint32_t ctx[20];                   // packed probability state per context
-    uint8_t mrow[64], mctx[64];         // refinement pass: rows and context codes per column
+// Label and probability tables of a CTA.
+struct EncTables {
+    uint8_t zc[4][256];   // zero-coding label x 4: left rows k-1..k+1 in bits 0-2, right 3-5, up 6, down 7
+    uint8_t sc[256];      // sign label x 4 | XOR bit: significance of left, right, up, down in bits 0-3, signs 4-7
+    uint2 next[94];       // context words after an MPS and after an LPS, by 2 x state + MPS
 };
+
+// A block's decisions of one stripe and pass (at most ten a column) and its
+// context words (Qe << 16 | (2 x state + MPS) << 3).
+struct EncState {
+    uint8_t sym[64 * 10 + 16];   // label x 4 | decision
+    uint32_t ctx[20];
+};
+
+__device__ __forceinline__ uint32_t enc_word(int state, int mps)
+{
+    return ((uint32_t)c_qe[state] << 16) | (uint32_t)((2 * state + mps) << 3);
+}
+
+__device__ void build_enc_tables(EncTables &t)
+{
+    for (int i = threadIdx.x; i < 94; i += blockDim.x) {
+        const int st = i >> 1, mps = i & 1, sw = st == 0 || st == 6 || st == 14;
+        t.next[i] = make_uint2(enc_word(c_nmps[st], mps), enc_word(c_nlps[st], mps ^ sw));
+    }
+    for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) {
+        const int b = i & 255;
+        auto bit = [&](int k) { return (b >> k) & 1; };
+        t.zc[i >> 8][b] = (uint8_t)(4 * zc_label(i >> 8, bit(1) + bit(4), bit(6) + bit(7),
+                                                 bit(0) + bit(2) + bit(3) + bit(5)));
+    }
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) {   // ISO Tables D.2/D.3
+        auto ctb = [&](int k) { return (i >> k) & 1 ? ((i >> (4 + k)) & 1 ? -1 : 1) : 0; };
+        int hc = ctb(0) + ctb(1), vc = ctb(2) + ctb(3);
+        hc = hc > 1 ? 1 : (hc < -1 ? -1 : hc);
+        vc = vc > 1 ? 1 : (vc < -1 ? -1 : vc);
+        const int cx = hc == 0 ? (vc == 0 ? 9 : 10) : 12 + hc * vc;
+        const int xr = hc == 0 ? vc < 0 : hc < 0;
+        t.sc[i] = (uint8_t)((4 * cx) | xr);
+    }
+}
 
 // Magnitude of sample (x, y) of block d: the int32 input, or the float input
 // quantised floor(|v| / step) (ISO E.2 deadzone).
@@ -50,9 +90,7 @@ __device__ __forceinline__ uint32_t magnitude(const tc_t1_enc_desc &d, const voi
     return (uint32_t)(v < 0 ? -(int64_t)v : v);
 }
 
-// MQ encoder (ISO C.2.1-C.2.9).  A is 16 bits wide as in the standard; each
-// context word is the decoder's packed state (Qe << 16 | NMPS << 1 |
-// NLPS << 7 | SWITCH << 13 | MPS).  The last byte emitted (B of the
+// MQ encoder (ISO C.2.1-C.2.9).  A is 16 bits wide as in the standard.  The last byte emitted (B of the
 // standard) stays in a register until the next one is emitted, since a
 // carry can still increment it; bytes before it are final.
 struct MQEnc {
@@ -110,34 +148,26 @@ struct MQEnc {
             }
         }
     }
-    __device__ __forceinline__ void renorm()
+    // One decision of the context whose word is w; returns its word afterwards.
+    __device__ __forceinline__ uint32_t encode(const EncTables &T, uint32_t w, uint32_t d)
     {
-        do {
-            a <<= 1;
-            c <<= 1;
-            if (--ct == 0) byteout();
-        } while ((a & 0x8000u) == 0u);
-    }
-    __device__ __forceinline__ void encode(uint32_t *ctx, const uint32_t *tbl, int cx, uint32_t d)
-    {
-        const uint32_t w = ctx[cx];
-        const uint32_t qe = w >> 16, mps = w & 1u;
-        a -= qe;
-        if (d == mps) {
-            if ((a & 0x8000u) == 0u) {
-                if (a < qe) a = qe;
-                else c += qe;
-                ctx[cx] = tbl[(w >> 1) & 63] | mps;
-                renorm();
-            } else {
-                c += qe;
-            }
-        } else {
-            if (a < qe) c += qe;
-            else a = qe;
-            ctx[cx] = tbl[(w >> 7) & 63] | (mps ^ ((w >> 13) & 1u));
-            renorm();
+        const uint2 succ = *reinterpret_cast<const uint2 *>(reinterpret_cast<const char *>(T.next) + (w & 0x3F8u));
+        const uint32_t qe = w >> 16, a1 = a - qe;
+        const bool lps = d != ((w >> 3) & 1u);
+        const bool upper = lps == (a1 < qe);   // the upper sub-interval (conditional exchange included)
+        a = upper ? a1 : qe;
+        c = upper ? c + qe : c;
+        int sh = __clz(a) - 16;
+        const uint32_t nx = sh ? (lps ? succ.y : succ.x) : w;
+        a <<= sh;
+        while (sh >= ct) {
+            c <<= ct;
+            sh -= ct;
+            byteout();
         }
+        c <<= sh;
+        ct -= sh;
+        return nx;
     }
     // FLUSH (ISO C.2.9); returns the codeword length (a final 0xFF dropped).
     __device__ __forceinline__ uint32_t flush()
@@ -161,199 +191,179 @@ struct MQEnc {
     }
 };
 
-// The first `limit` coding passes of a block whose state S holds the signs
-// and a cleared coding state (the lanes in lock-step; limit is the same in
-// every lane, so the early exits are uniform).
-__device__ void encode_block(EncState &S, const Tables &T, MQEnc &mq, const tc_t1_enc_desc &d, const void *in,
-                             int numbps, int limit, int lane)
-{
-    const int w = d.w, h = d.h, orient = d.orient;
-    uint32_t *ctx = S.ctx;
-    const uint32_t *tbl = T.mq;
-    const uint8_t *zc = T.zc[orient];
-    uint32_t *F = S.F;
-    const int nstripes = (h + 3) >> 2;
-    constexpr int G = 32, CPL = 2;
-    const unsigned gmask = 0xffffffffu;
-    auto bit = [&](int y, int c, int) -> uint32_t { return (uint32_t)(S.bits[c] >> y) & 1u; };
-    auto sign_bit = [&](int y, int c) -> uint32_t { return (uint32_t)(S.neg[c] >> y) & 1u; };
+constexpr unsigned kAll = 0xffffffffu;
 
-    int done = 0;  // coding passes emitted
-    for (int p = numbps - 1; p >= 0 && done < limit; --p) {
-        // this bit-plane's bits, the lanes' columns
-#pragma unroll
-        for (int j = 0; j < CPL; j++) {
-            const int c = lane + G * j;
-            unsigned long long m = 0;
-            if (c < w)
-                for (int y = 0; y < h; y++) m |= (unsigned long long)((magnitude(d, in, c, y) >> p) & 1u) << y;
-            S.bits[c] = m;
+// The first `limit` coding passes of a block.  neg: the lane's columns' signs.
+__device__ void encode_block(EncState &S, const EncTables &T, MQEnc &mq, const tc_t1_enc_desc &d, const void *in,
+                             const unsigned long long (&neg)[2], int numbps, int limit, int lane)
+{
+    const int w = d.w, h = d.h, nstripes = (h + 3) >> 2;
+    const uint8_t *zc = T.zc[d.orient];
+    char *ctxb = reinterpret_cast<char *>(S.ctx);
+    auto ctx_at = [&](uint32_t sym) -> uint32_t & { return *reinterpret_cast<uint32_t *>(ctxb + (sym & 0x7Cu)); };
+    unsigned long long sig[2] = {0ull, 0ull}, pi[2] = {0ull, 0ull}, ref[2] = {0ull, 0ull}, bits[2] = {0ull, 0ull};
+    // six rows, -1..4, of stripe s of a column
+    auto window = [](unsigned long long m, int s) -> uint32_t {
+        return (uint32_t)(s ? m >> (4 * s - 1) : m << 1) & 63u;
+    };
+    auto spread3 = [](uint32_t x) -> uint32_t { return (x | (x >> 1) | (x >> 2)) & 15u; };   // rows k-1..k+1 of a window
+
+    // the list through the MQ coder
+    auto run_list = [&](int n) {
+        if (n == 0) return;
+        __syncwarp();
+        uint32_t s0 = S.sym[0];
+        uint32_t cw = ctx_at(s0);
+        for (int i = 1;; i++) {
+            const uint32_t s1 = S.sym[i];   // one past the end for the last
+            const uint32_t cn = ctx_at(s1);
+            const uint32_t nx = mq.encode(T, cw, s0 & 1u);
+            ctx_at(s0) = nx;
+            if (i >= n) break;
+            cw = ((s0 ^ s1) & 0x7Cu) ? cn : nx;
+            s0 = s1;
         }
         __syncwarp();
-        if (p != numbps - 1) {
-            // ---- significance propagation pass (ISO D.3.1) ----
-            for (int s = 0; s < nstripes; s++) {
-                const int rows = min(4, h - 4 * s);
-                __syncwarp();
-                bool any[CPL];
-#pragma unroll
-                for (int j = 0; j < CPL; j++) {
-                    const int c = lane + G * j;
-                    bool a = false;
-                    if (c < w) {
-                        const uint32_t f = F[s * 64 + c];
-                        for (int k = 0; k < rows; k++) a |= !(f & self_bit(k)) && ((f >> (3 * k)) & 0x1EFu);
-                    }
-                    any[j] = a;
-                }
-                unsigned long long cand = group_ballot<G>(any, gmask, 0);
-                while (cand) {
-                    const int c = __ffsll((long long)cand) - 1;
-                    cand &= cand - 1;
-                    uint32_t f = F[s * 64 + c];
-                    const uint32_t f0 = f;
-                    for (int k = 0; k < rows; k++) {
-                        if (f & self_bit(k)) continue;
-                        const uint32_t n9 = (f >> (3 * k)) & 0x1FFu;
-                        if (!(n9 & 0x1EFu)) continue;
-                        f |= pi_bit(k);
-                        const int y = 4 * s + k;
-                        const uint32_t b = bit(y, c, p);
-                        mq.encode(ctx, tbl, zc[n9], b);
-                        if (b) {
-                            const uint32_t si = T.sc[sign_index(S.sgn, n9, c, y)];
-                            const uint32_t neg = sign_bit(y, c);
-                            mq.encode(ctx, tbl, si & 15, neg ^ (si >> 4));
-                            f |= self_bit(k);
-                            mark_significant(F, S.sgn, s, k, c, w, nstripes, neg);
-                            if (c + 1 < w) cand |= 1ull << (c + 1);  // the next column gained a neighbour
-                        }
-                    }
-                    if (f != f0) F[s * 64 + c] = f;
-                }
-            }
-            if (++done >= limit) break;
+    };
 
-            // ---- magnitude refinement pass (ISO D.3.3) ----
-            for (int s = 0; s < nstripes; s++) {
-                const int rows = min(4, h - 4 * s);
-                __syncwarp();
-                bool any[CPL];
+    int p = numbps - 1, type = 0;   // 0 cleanup, 1 significance propagation, 2 refinement
+    for (int done = 0; done < limit; done++) {
+        if (type == 1 || done == 0) {
+            // this bit-plane's bits
 #pragma unroll
-                for (int j = 0; j < CPL; j++) {
-                    const int c = lane + G * j;
-                    uint32_t rr = 0, codes = 0;
-                    if (c < w) {
-                        const uint32_t f = F[s * 64 + c];
-                        for (int k = 0; k < rows; k++) {
-                            if ((f & self_bit(k)) && !(f & pi_bit(k))) {
-                                rr |= 1u << k;
-                                const uint32_t code = (f & ref_bit(k)) ? 2u : (((f >> (3 * k)) & 0x1EFu) ? 1u : 0u);
-                                codes |= code << (2 * k);
-                            }
-                        }
-                        S.mrow[c] = (uint8_t)rr;
-                        S.mctx[c] = (uint8_t)codes;
-                        if (rr) F[s * 64 + c] = f | (rr << 22);
-                    }
-                    any[j] = rr != 0;
+            for (int j = 0; j < 2; j++) {
+                unsigned long long m = 0;
+                if (lane + 32 * j < w) {
+#pragma unroll 8
+                    for (int y = 0; y < h; y++)
+                        m |= (unsigned long long)((magnitude(d, in, lane + 32 * j, y) >> p) & 1u) << y;
                 }
-                unsigned long long cand = group_ballot<G>(any, gmask, 0);
-                __syncwarp();
-                while (cand) {
-                    const int c = __ffsll((long long)cand) - 1;
-                    cand &= cand - 1;
-                    uint32_t rr = S.mrow[c];
-                    const uint32_t codes = S.mctx[c];
-                    while (rr) {
-                        const int k = __ffs(rr) - 1;
-                        rr &= rr - 1;
-                        mq.encode(ctx, tbl, 14 + ((codes >> (2 * k)) & 3u), bit(4 * s + k, c, p));
-                    }
-                }
+                bits[j] = m;
+                pi[j] = 0ull;
             }
-            if (++done >= limit) break;
         }
-
-        // ---- cleanup pass (ISO D.3.4) ----
         for (int s = 0; s < nstripes; s++) {
             const int rows = min(4, h - 4 * s);
-            const uint32_t rmask = (1u << rows) - 1u;
-            __syncwarp();
-            bool any[CPL];
+            const uint32_t rowmask = (1u << rows) - 1u;
+            // windows of the lane's columns: significance in bits 0-5, signs in 6-11
+            const uint32_t v0 = window(sig[0], s) | (window(neg[0], s) << 6);
+            const uint32_t v1 = window(sig[1], s) | (window(neg[1], s) << 6);
+            int n = 0;                 // decisions in the list
+            uint32_t carry = 0;        // column 31's new samples, for column 32
 #pragma unroll
-            for (int j = 0; j < CPL; j++) {
-                const int c = lane + G * j;
-                bool a = false;
-                if (c < w) {
-                    const uint32_t f = F[s * 64 + c];
-                    uint32_t done = (f >> 18) & 0xFu;  // pi
+            for (int j = 0; j < 2; j++) {
+                if (32 * j >= w) break;
+                const uint32_t v = j ? v1 : v0;
+                uint32_t lv = __shfl_up_sync(kAll, v, 1), rv = __shfl_down_sync(kAll, v, 1);
+                const uint32_t edge = j ? __shfl_sync(kAll, v0, 31) : __shfl_sync(kAll, v1, 0);
+                if (lane == 0) lv = j ? edge : 0u;
+                if (lane == 31) rv = j ? 0u : edge;
+                const uint32_t own = v & 63u, right = rv & 63u;
+                const uint32_t here = (own >> 1) & 15u;                       // the stripe's significant samples
+                const uint32_t b = (uint32_t)(bits[j] >> (4 * s)) & 15u;
+                const uint32_t mask = lane + 32 * j < w ? rowmask : 0u;
+                const uint32_t near = spread3(lv & 63u) | spread3(right) | ((own | (own >> 2)) & 15u);
+
+                if (type == 2) {
+                    // ---- magnitude refinement (ISO D.3.3) ----
+                    const uint32_t m = here & ~(uint32_t)(pi[j] >> (4 * s)) & mask;
+                    const uint32_t r = (uint32_t)(ref[j] >> (4 * s)) & 15u;
+                    int at = __popc(m), sum = at;
 #pragma unroll
-                    for (int k = 0; k < 4; k++) done |= ((f >> (3 * k + 4)) & 1u) << k;
-                    a = (~done & rmask) != 0u;
-                }
-                any[j] = a;
-            }
-            unsigned long long cand = group_ballot<G>(any, gmask, 0);
-            while (cand) {
-                const int c = __ffsll((long long)cand) - 1;
-                cand &= cand - 1;
-                uint32_t f = F[s * 64 + c];
-                const uint32_t f0 = f;
-                int k = 0;
-                if (rows == 4 && (f & kSigMask) == 0u) {
-                    // run-length mode: four rows with an all-zero neighbourhood
-                    const uint32_t four = (uint32_t)(S.bits[c] >> (4 * s)) & 0xFu;
-                    const int r = four ? __ffs(four) - 1 : -1;
-                    if (r < 0) {
-                        mq.encode(ctx, tbl, 18, 0u);
-                        continue;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int u = __shfl_up_sync(kAll, sum, o);
+                        if (lane >= o) sum += u;
                     }
-                    mq.encode(ctx, tbl, 18, 1u);
-                    mq.encode(ctx, tbl, 17, (uint32_t)(r >> 1));
-                    mq.encode(ctx, tbl, 17, (uint32_t)(r & 1));
-                    const int y = 4 * s + r;
-                    const uint32_t si = T.sc[sign_index(S.sgn, (f >> (3 * r)) & 0x1FFu, c, y)];
-                    const uint32_t neg = sign_bit(y, c);
-                    mq.encode(ctx, tbl, si & 15, neg ^ (si >> 4));
-                    f |= self_bit(r);
-                    mark_significant(F, S.sgn, s, r, c, w, nstripes, neg);
-                    k = r + 1;
+                    at = n + sum - at;
+                    n += __shfl_sync(kAll, sum, 31);
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if ((m >> k) & 1u)
+                            S.sym[at++] = (uint8_t)(((r >> k) & 1u ? 64u : ((near >> k) & 1u ? 60u : 56u)) | ((b >> k) & 1u));
+                    ref[j] |= (unsigned long long)m << (4 * s);
+                    continue;
                 }
-                for (; k < rows; k++) {
-                    if (f & (self_bit(k) | pi_bit(k))) continue;
-                    const uint32_t n9 = (f >> (3 * k)) & 0x1FFu;
-                    const int y = 4 * s + k;
-                    const uint32_t b = bit(y, c, p);
-                    mq.encode(ctx, tbl, zc[n9], b);
+
+                const uint32_t avail = ~here & mask;
+                uint32_t m, left_new;   // samples coded; the left column's new ones
+                if (type == 1) {
+                    // ---- significance propagation (ISO D.3.1) ----
+                    m = avail & near;
+                    left_new = lane == 0 ? carry : 0u;
+                    for (;;) {
+                        m |= avail & (left_new | (left_new << 1) | (left_new >> 1));
+                        m |= avail & ((m & b) << 1);
+                        m |= avail & ((m & b) << 1);
+                        m |= avail & ((m & b) << 1);
+                        const uint32_t l = __shfl_up_sync(kAll, m & b, 1);
+                        const uint32_t now = lane == 0 ? carry : l;
+                        const bool changed = now != left_new;
+                        left_new = now;
+                        if (!__any_sync(kAll, changed)) break;
+                    }
+                    pi[j] |= (unsigned long long)m << (4 * s);
+                } else {
+                    // ---- cleanup (ISO D.3.4) ----
+                    m = avail & ~(uint32_t)(pi[j] >> (4 * s));
+                    const uint32_t l = __shfl_up_sync(kAll, m & b, 1);
+                    left_new = lane == 0 ? carry : l;
+                }
+                const uint32_t fresh = m & b;
+                carry = __shfl_sync(kAll, fresh, 31);
+                if (type == 1 && !__any_sync(kAll, m != 0u)) continue;
+                const uint32_t left = (lv & 63u) | (left_new << 1), up = own | (fresh << 1);
+                // run-length column: four rows, nothing significant around
+                const bool run = type == 0 && rows == 4 && mask && (own | left | right) == 0u;
+                const int first = run ? (b ? __ffs((int)b) - 1 : 4) : -1;   // its first significant row
+                int at = run ? (b ? 4 + 3 - first + __popc(b >> (first + 1)) : 1) : __popc(m) + __popc(fresh), sum = at;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(kAll, sum, o);
+                    if (lane >= o) sum += u;
+                }
+                at = n + sum - at;
+                n += __shfl_sync(kAll, sum, 31);
+                if (run) {
+                    S.sym[at++] = (uint8_t)(kSymRun | (b != 0u));
                     if (b) {
-                        const uint32_t si = T.sc[sign_index(S.sgn, n9, c, y)];
-                        const uint32_t neg = sign_bit(y, c);
-                        mq.encode(ctx, tbl, si & 15, neg ^ (si >> 4));
-                        f |= self_bit(k);
-                        mark_significant(F, S.sgn, s, k, c, w, nstripes, neg);
+                        S.sym[at++] = (uint8_t)(kSymUni | (first >> 1));
+                        S.sym[at++] = (uint8_t)(kSymUni | (first & 1));
                     }
                 }
-                if (f != f0) F[s * 64 + c] = f;
+                const uint32_t ln = lv >> 6, rn = rv >> 6, on = v >> 6;   // signs
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (((m >> k) & 1u) && k > first)
+                        S.sym[at++] = (uint8_t)(zc[((left >> k) & 7u) | (((right >> k) & 7u) << 3) | (((up >> k) & 1u) << 6) |
+                                                   (((own >> (k + 2)) & 1u) << 7)] |
+                                                ((b >> k) & 1u));
+                    if (((fresh >> k) & 1u) && k >= first) {
+                        const uint32_t i = ((left >> (k + 1)) & 1u) | (((right >> (k + 1)) & 1u) << 1) |
+                                           (((up >> k) & 1u) << 2) | (((own >> (k + 2)) & 1u) << 3) |
+                                           (((ln >> (k + 1)) & 1u) << 4) | (((rn >> (k + 1)) & 1u) << 5) |
+                                           (((on >> k) & 1u) << 6) | (((on >> (k + 2)) & 1u) << 7);
+                        S.sym[at++] = (uint8_t)(T.sc[i] ^ ((on >> (k + 1)) & 1u));
+                    }
+                }
+                sig[j] |= (unsigned long long)fresh << (4 * s);
             }
+            run_list(n);
         }
-        ++done;
-        __syncwarp();
-        for (int i = lane; i < nstripes * 64; i += G) F[i] &= ~0x3C0000u;  // clear pi
-        __syncwarp();
+        if (type == 0) --p;
+        type = type == 0 ? 1 : (type == 1 ? 2 : 0);
     }
 }
 
 // One code-block per warp; blocks b = blockIdx.x * kEncWarps + warp.
-__global__ void __launch_bounds__(32 * kEncWarps)
+__global__ void __launch_bounds__(32 * kEncWarps, 6)
     t1_encode_kernel(const tc_t1_enc_desc *__restrict__ desc, int n, const void *__restrict__ in,
                      uint8_t *__restrict__ out, uint32_t cap, tc_t1_enc_result *__restrict__ res)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    Tables &T = *reinterpret_cast<Tables *>(smem);
+    __shared__ EncTables T;
+    __shared__ EncState states[kEncWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    EncState &S = reinterpret_cast<EncState *>(smem + ((sizeof(Tables) + 15) & ~size_t(15)))[warp];
-    build_tables(T);
+    EncState &S = states[warp];
+    build_enc_tables(T);
     __syncthreads();
     const int bi = blockIdx.x * kEncWarps + warp;
     if (bi >= n) return;
@@ -368,9 +378,10 @@ __global__ void __launch_bounds__(32 * kEncWarps)
     // largest magnitude and the signs, rows coalesced across the lanes
     const bool irrev = (d.flags & TC_CBLK_IRREVERSIBLE) != 0;
     uint32_t mx = 0;
-    unsigned long long neg0 = 0, neg1 = 0;  // columns lane and lane + 32
+    unsigned long long neg[2] = {0ull, 0ull};  // columns lane and lane + 32
     for (int y = 0; y < h; y++) {
         const size_t row = d.in_off + (size_t)y * d.in_pitch;
+#pragma unroll
         for (int j = 0; j < 2; j++) {
             const int x = lane + 32 * j;
             if (x >= w) continue;
@@ -378,17 +389,11 @@ __global__ void __launch_bounds__(32 * kEncWarps)
             const bool ng = irrev ? static_cast<const float *>(in)[row + x] < 0.0f
                                   : static_cast<const int32_t *>(in)[row + x] < 0;
             mx = max(mx, m);
-            if (ng && m) (j ? neg1 : neg0) |= 1ull << y;
+            if (ng && m) neg[j] |= 1ull << y;
         }
     }
-    S.neg[lane] = neg0;
-    S.neg[lane + 32] = neg1;
-    for (int i = lane; i < kMaxStripes * 64; i += 32) S.F[i] = 0u;
-    for (int i = lane; i < kSgnCols; i += 32) S.sgn[i] = 0ull;
-    for (int i = lane; i < 19; i += 32) {
-        const int st = i == 0 ? 4 : (i == 17 ? 46 : (i == 18 ? 3 : 0));
-        S.ctx[i] = T.mq[st];
-    }
+    if (lane < 19) S.ctx[lane] = enc_word(lane == 0 ? 4 : (lane == 17 ? 46 : (lane == 18 ? 3 : 0)), 0);
+    for (int i = lane; i < (int)sizeof S.sym; i += 32) S.sym[i] = 0;   // one past a list is read, too
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     __syncwarp();
@@ -401,7 +406,7 @@ __global__ void __launch_bounds__(32 * kEncWarps)
         const int limit = d.max_passes && d.max_passes < total ? (int)d.max_passes : total;
         MQEnc mq;
         mq.init(out + (size_t)bi * cap, cap, lane == 0);
-        encode_block(S, T, mq, d, in, numbps, limit, lane);
+        encode_block(S, T, mq, d, in, neg, numbps, limit, lane);
         r.len = mq.flush();
         r.passes = (uint32_t)limit;
         if (mq.overflow || r.len > cap) {
@@ -413,18 +418,13 @@ __global__ void __launch_bounds__(32 * kEncWarps)
     if (lane == 0) res[bi] = r;
 }
 
-constexpr size_t kEncSmem = ((sizeof(Tables) + 15) & ~size_t(15)) + kEncWarps * sizeof(EncState);
-
 }  // namespace
 
 cudaError_t launch_t1_encode(tc_ctx *ctx, const tc_t1_enc_desc *d_desc, int n, const void *d_in, uint8_t *d_out,
                              uint32_t cap, tc_t1_enc_result *d_res)
 {
     if (n <= 0) return cudaSuccess;
-    static DeviceFlags attr;
-    if (cudaError_t e = set_smem_once(attr, ctx->device, t1_encode_kernel, kEncSmem)) return e;
-    t1_encode_kernel<<<(n + kEncWarps - 1) / kEncWarps, 32 * kEncWarps, kEncSmem, ctx->stream>>>(d_desc, n, d_in, d_out,
-                                                                                               cap, d_res);
+    t1_encode_kernel<<<(n + kEncWarps - 1) / kEncWarps, 32 * kEncWarps, 0, ctx->stream>>>(d_desc, n, d_in, d_out, cap, d_res);
     ctx->launches++;
     return cudaGetLastError();
 }
