@@ -894,7 +894,7 @@ static int dwt_forward(tc_ctx *ctx, int wavelet, int rounding, const void *d_in,
             io.out[0] = static_cast<char *>(ctx->scratch.ptr) + ((l - 1) & 1) * slab;
             io.out_pitch = ws[1];
         }
-        e = launch_fdwt_level(ctx, io, wavelet, rounding);
+        e = launch_fdwt_level(ctx, io, wavelet, rounding, l > 1);
         if (e != cudaSuccess) return cuda_status(ctx, e, "forward DWT");
         src = io.out[0];
         sp = io.out_pitch;

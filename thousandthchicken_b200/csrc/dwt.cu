@@ -16,6 +16,13 @@
 //     de-interleaved;
 //   * the store writes each row's low and high halves to the level's LL and
 //     HL (even rows) or LH and HH (odd rows) bands, coalesced.
+// The odd row stride keeps the row walk of the horizontal pass free of bank
+// conflicts, a lane's (mirrored) columns are worked out once, a thread's store
+// stays in one band, and the levels are chained with programmatic dependent
+// launch (not the first: its early CTAs would crowd out the previous
+// transform's last levels, 2048x2048 81 against 56 us).  Five levels of
+// 2999x2001 5/3 68 -> 33 us, six of 4096x4096 9/7 130 -> 69 us (1.9 TB/s of
+// level traffic); the rest is the levels of 512x512 and less, 4 to 5 us each.
 // 5/3 uses floor (ISO) or truncating (reference, defect D13) rounding; 9/7
 // uses fp32 with the scaling factors applied as floats (defects D10-D12
 // fixed).  The lifting steps and their order follow ISO F.4.8.
@@ -40,7 +47,7 @@ struct FwdGeo {
     static constexpr int TY = NR - 2 * H;         // output rows per tile
     static constexpr int TX = 120;                // output columns per tile (even)
     static constexpr int NC = TX + 2 * H;         // extended columns
-    static constexpr int S = (NC % 8 == 4) ? NC : NC + 4;  // row stride, S/4 odd
+    static constexpr int S = NC + 1;              // row stride, odd: threads on consecutive rows hit different banks
     static constexpr int SEG = 30;                // outputs per row segment (even)
     static constexpr int SEGN = SEG + 2 * H;      // inputs per row segment
     static constexpr int VN = 32 + H;             // rows lifted by one thread of a column pair
@@ -97,16 +104,20 @@ __global__ void __launch_bounds__(kThreads) fdwt_level_kernel(LevelIO io)
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
     const int w = io.w, h = io.h;
     const T *in = static_cast<const T *>(io.ll[c]);
+    pdl_allow_next();
+    pdl_wait_prev();
 
-    // 1. stage the extended tile
-    const bool interior = x0 >= H && x0 - H + NC <= w && y0 >= H && y0 - H + NR <= h;
+    // 1. stage the extended tile; a lane's columns are the same in every row
+    constexpr int kCols = (NC + 31) / 32;
+    int xo[kCols];
+#pragma unroll
+    for (int j = 0; j < kCols; j++) xo[j] = lane + 32 * j < NC ? mirror(x0 - H + lane + 32 * j, w) : -1;
+#pragma unroll 2
     for (int r = warp; r < NR; r += kThreads / 32) {
-        const int y = interior ? y0 - H + r : mirror(y0 - H + r, h);
-        const T *row = in + (size_t)y * io.ll_pitch;
-        for (int e = lane; e < NC; e += 32) {
-            const int x = interior ? x0 - H + e : mirror(x0 - H + e, w);
-            cp_async4(t + r * S + e, row + x);
-        }
+        const T *row = in + (size_t)mirror(y0 - H + r, h) * io.ll_pitch;
+#pragma unroll
+        for (int j = 0; j < kCols; j++)
+            if (xo[j] >= 0) cp_async4(t + r * S + lane + 32 * j, row + xo[j]);
     }
     cp_async_wait_all();
     __syncthreads();
@@ -155,51 +166,53 @@ __global__ void __launch_bounds__(kThreads) fdwt_level_kernel(LevelIO io)
 
     // 4. store: row by row, the low half to LL / LH, the high half to HL / HH;
     //    a thread keeps one of the 120 output slots of a row (60 low, 60 high)
-    //    and walks every other row
+    //    and walks every other row, so it stays in one band
     const int wl = (w + 1) >> 1, hl = (h + 1) >> 1;
     constexpr int HALF = TX / 2;
-    const int j = tid % 128, r0 = tid / 128;
+    const int j = tid % 128, odd = tid / 128;
     if (j < TX) {
         const bool hi = j >= HALF;
         const int i = hi ? j - HALF : j;
         const int x = x0 + 2 * i + (hi ? 1 : 0);
         if (x < w) {
-            const int xb = (x0 >> 1) + i;
-            T *ll = static_cast<T *>(io.out[c]) + xb;
-            T *bands = static_cast<T *>(io.bands[c]) + xb + (hi ? wl : 0);
-            const T *src = t + (hi ? 64 : 0) + i;
-            for (int r = r0; r < TY && y0 + r < h; r += 2) {
-                const int y = y0 + r, yb = y >> 1;
-                const T val = src[(H + r) * S];
-                if (y & 1) bands[(size_t)(hl + yb) * io.bands_pitch] = val;
-                else if (hi) bands[(size_t)yb * io.bands_pitch] = val;
-                else ll[(size_t)yb * io.out_pitch] = val;
-            }
+            const int xb = (x0 >> 1) + i, yb = y0 >> 1;
+            const bool ll = !odd && !hi;
+            const size_t pitch = ll ? (size_t)io.out_pitch : (size_t)io.bands_pitch;
+            T *dst = static_cast<T *>(ll ? io.out[c] : io.bands[c]) + (size_t)(odd ? hl + yb : yb) * pitch + xb + (hi ? wl : 0);
+            const T *src = t + (H + odd) * S + (hi ? 64 : 0) + i;
+            const int n = (min(TY, h - y0) - odd + 1) >> 1;
+#pragma unroll 4
+            for (int k = 0; k < n; k++, dst += pitch, src += 2 * S) *dst = *src;
         }
     }
 }
 
 template <typename T, int WAVELET, int RND>
-cudaError_t run_fdwt(tc_ctx *ctx, const LevelIO &io)
+cudaError_t run_fdwt(tc_ctx *ctx, const LevelIO &io, bool chained)
 {
     using G = FwdGeo<WAVELET>;
     constexpr size_t smem = (size_t)G::NR * G::S * sizeof(T);
     static DeviceFlags attr;
     if (cudaError_t e = set_smem_once(attr, ctx->device, fdwt_level_kernel<T, WAVELET, RND>, smem)) return e;
     dim3 grid((io.w + G::TX - 1) / G::TX, (io.h + G::TY - 1) / G::TY, io.ncomp);
-    fdwt_level_kernel<T, WAVELET, RND><<<grid, kThreads, smem, ctx->stream>>>(io);
+    if (chained) {
+        if (cudaError_t e = launch_pdl(fdwt_level_kernel<T, WAVELET, RND>, grid, dim3(kThreads), smem, ctx->stream, io))
+            return e;
+    } else {
+        fdwt_level_kernel<T, WAVELET, RND><<<grid, kThreads, smem, ctx->stream>>>(io);
+    }
     ctx->launches++;
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_fdwt_level(tc_ctx *ctx, const LevelIO &io, int wavelet, int rounding)
+cudaError_t launch_fdwt_level(tc_ctx *ctx, const LevelIO &io, int wavelet, int rounding, bool chained)
 {
     if (io.w <= 0 || io.h <= 0) return cudaSuccess;
-    if (wavelet) return run_fdwt<float, 1, 0>(ctx, io);
-    if (rounding == TC_ROUND_TRUNC) return run_fdwt<int32_t, 0, TC_ROUND_TRUNC>(ctx, io);
-    return run_fdwt<int32_t, 0, TC_ROUND_FLOOR>(ctx, io);
+    if (wavelet) return run_fdwt<float, 1, 0>(ctx, io, chained);
+    if (rounding == TC_ROUND_TRUNC) return run_fdwt<int32_t, 0, TC_ROUND_TRUNC>(ctx, io, chained);
+    return run_fdwt<int32_t, 0, TC_ROUND_FLOOR>(ctx, io, chained);
 }
 
 }  // namespace tc

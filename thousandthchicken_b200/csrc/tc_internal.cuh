@@ -222,7 +222,9 @@ void rev_tile_shape(int wavelet, int *tx, int *ty);
 // writing out_type samples of `bits` bits.
 cudaError_t launch_idwt_batch(tc_ctx *ctx, const RevJob *d_jobs, int njobs, int ntiles, int wavelet, int rounding,
                               int color, int ncomp, int out_type, int bits);
-cudaError_t launch_fdwt_level(tc_ctx *ctx, const LevelIO &io, int wavelet, int rounding);
+// chained: the previous kernel on the stream is the level before (the launch
+// may be scheduled while it finishes).
+cudaError_t launch_fdwt_level(tc_ctx *ctx, const LevelIO &io, int wavelet, int rounding, bool chained);
 
 // Last reverse 9/7 level of a three-component image with the inverse ICT
 // fused in, packed fp32x2 lifting (dwt_rev97.cu).  rev97_handles says
