@@ -125,7 +125,53 @@ __device__ __forceinline__ void rev_stage(const LevelIO &io, int bx, int by, int
         T *t = tiles + cc * NR * S;
         const T *ll = static_cast<const T *>(io.ll[cbase + cc]);
         const T *coef = static_cast<const T *>(io.coef[cbase + cc]);
-        if (interior) {
+        // Four samples of a row are two of the low and two of the high band:
+        // where the bands' rows are 8-byte aligned, two 8-byte loads and one
+        // 16-byte store (5/3, whose tile starts two columns after such a quad:
+        // two 8-byte stores) instead of four 4-byte copies, all loads in
+        // flight at once.  Five reverse levels of 2048x2048: 9/7 35.1 -> 27.6
+        // us, 5/3 34.8 -> 28.3; six of 4096x4096: 66.8 -> 62.4 and 68 -> 59 us.
+        constexpr int SH = H % 4;   // columns of the first quad before the tile
+        const bool pairs = interior && x0 + TX + H + SH <= w && ((wl | io.ll_pitch | io.coef_pitch) & 1) == 0 &&
+                           ((reinterpret_cast<uintptr_t>(ll) | reinterpret_cast<uintptr_t>(coef)) & 7) == 0;
+        if (pairs) {
+            using V2 = typename std::conditional<std::is_same<T, float>::value, float2, int2>::type;
+            const int xs = (x0 - H - SH) >> 1;
+            auto rows = [&](int r, const T *&lo, const T *&hi) {
+                const int y = y0 - H + r, yb = y >> 1;
+                lo = ((y & 1) ? coef + (size_t)(hl + yb) * io.coef_pitch : ll + (size_t)yb * io.ll_pitch) + xs;
+                hi = coef + (size_t)((y & 1) ? hl + yb : yb) * io.coef_pitch + wl + xs;
+            };
+            auto store = [&](int r, int q, const V2 &lo, const V2 &hi) {
+                T *d = t + r * S + 4 * q - SH;
+                if constexpr (SH == 0) {
+                    *reinterpret_cast<Vec4<T> *>(d) = Vec4<T>{lo.x, hi.x, lo.y, hi.y};
+                } else {
+                    if (q > 0) *reinterpret_cast<V2 *>(d) = V2{lo.x, hi.x};
+                    if (4 * q < NC) *reinterpret_cast<V2 *>(d + 2) = V2{lo.y, hi.y};
+                }
+            };
+            constexpr int RSTEP = kThreads / 32, RN = NR / RSTEP, EXTRA = (NC + 2 * SH) / 4 - 32;
+            static_assert((NC + 2 * SH) % 4 == 0 && EXTRA > 0 && NR * EXTRA <= kThreads, "quads of a tile");
+            V2 a[RN], b[RN], ea{}, eb{};
+#pragma unroll
+            for (int i = 0; i < RN; i++) {
+                const T *lo, *hi;
+                rows(warp + RSTEP * i, lo, hi);
+                a[i] = *reinterpret_cast<const V2 *>(lo + 2 * lane);
+                b[i] = *reinterpret_cast<const V2 *>(hi + 2 * lane);
+            }
+            const int er = tid / EXTRA, eq = 32 + tid % EXTRA;   // the row's last quads
+            if (er < NR) {
+                const T *lo, *hi;
+                rows(er, lo, hi);
+                ea = *reinterpret_cast<const V2 *>(lo + 2 * eq);
+                eb = *reinterpret_cast<const V2 *>(hi + 2 * eq);
+            }
+#pragma unroll
+            for (int i = 0; i < RN; i++) store(warp + RSTEP * i, lane, a[i], b[i]);
+            if (er < NR) store(er, eq, ea, eb);
+        } else if (interior) {
             // y0 - H is even and a warp's rows step by 8: a warp copies rows
             // of one parity only, so each lane's source is one band row
             // advancing by 4 rows of its plane per step
@@ -148,15 +194,19 @@ __device__ __forceinline__ void rev_stage(const LevelIO &io, int bx, int by, int
                 if (lane < NC % 32) cp_async4(dst + 32 * (NC / 32), src + 16 * (NC / 32));
             }
         } else {
+            // a lane's columns are the same in every row
+            constexpr int kCols = (NC + 31) / 32;
+            int xo[kCols];
+#pragma unroll
+            for (int j = 0; j < kCols; j++) xo[j] = lane + 32 * j < NC ? mirror(x0 - H + lane + 32 * j, w) : -1;
+#pragma unroll 2
             for (int r = warp; r < NR; r += kThreads / 32) {
                 const int my = mirror(y0 - H + r, h), yb = my >> 1;
                 const T *lrow = (my & 1) ? coef + (size_t)(hl + yb) * io.coef_pitch : ll + (size_t)yb * io.ll_pitch;
                 const T *hrow = coef + (size_t)((my & 1) ? hl + yb : yb) * io.coef_pitch + wl;
 #pragma unroll
-                for (int e = lane; e < NC; e += 32) {
-                    const int mx = mirror(x0 - H + e, w);
-                    cp_async4(t + r * S + e, ((mx & 1) ? hrow : lrow) + (mx >> 1));
-                }
+                for (int j = 0; j < kCols; j++)
+                    if (xo[j] >= 0) cp_async4(t + r * S + lane + 32 * j, ((xo[j] & 1) ? hrow : lrow) + (xo[j] >> 1));
             }
         }
     }
@@ -311,8 +361,10 @@ __device__ __forceinline__ void rev_tile(const LevelIO &io, int bits, int bx, in
 
 // One level of one image: tiles (blockIdx.x, blockIdx.y), one component per
 // blockIdx.z for plane levels.
+// Four plane CTAs per SM (64 registers): without the bound 5/3 took more and
+// three, 2048x2048 in two waves (38 against 28 us); five spill (34 us).
 template <typename T, int WAVELET, int RND, int NCOMP, int COLOR, typename OT>
-__global__ void __launch_bounds__(kThreads) idwt_rev_kernel(LevelIO io, int bits)
+__global__ void __launch_bounds__(kThreads, COLOR < 0 ? 4 : 1) idwt_rev_kernel(LevelIO io, int bits)
 {
     pdl_allow_next();
     pdl_wait_prev();
