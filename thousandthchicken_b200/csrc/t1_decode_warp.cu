@@ -47,10 +47,11 @@ constexpr int kLabRun = 72, kLabUni = 68;   // context labels are kept as byte o
 constexpr int kMaxSlots = 12;    // code-blocks per CTA at most
 // Launches of fewer blocks per SM than this decode Deep: the label of the
 // sample after the next is loaded too and one branch leaves the straight line,
-// more instructions but shorter waits.  768x768x3 lossy (3 blocks per SM) 1.88
-// -> 1.66 ms, 1024x1024x3 (5) 2.1 -> 1.92 ms; 1536x1536x3 (12) 2.25 against
-// 2.29 ms, 4096x4096x3 13.3 against 13.8 ms.
-constexpr int kDeepBlocks = 6;
+// more instructions but shorter waits.  Against the other kernel: 1024x1024x3
+// lossy (5 blocks per SM) 1.85 and 2.05 ms, 2048x2048 16-bit lossless (7) 5.1
+// and 5.7, 1920x1080x3 lossy (12) 2.3 and 2.4; 1792x1792x3 lossy (16) 3.4 and
+// 3.2, 4096x4096x3 13.9 and 13.3.
+constexpr int kDeepBlocks = 13;
 
 // Label and probability tables of a CTA.
 struct WarpTables {
@@ -797,15 +798,23 @@ t1_decode_warp_kernel(const tc_cblk_desc *__restrict__ desc, BlockQueue queue, i
     WarpTables &T = *reinterpret_cast<WarpTables *>(smem);
     build_warp_tables(T);
     __syncthreads();
-    const int lane = threadIdx.x & 31, slot = threadIdx.x >> 5;
+    // A warp's slot, alternately up and down the SM's four schedulers, so that
+    // the first (longest) blocks share theirs with the shortest or with none.
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = (warp & 4) ? warp ^ 3 : warp;
     if (slot >= slots) return;
     const size_t stride = sizeof(BlockState) + (size_t)np * kPlaneWords * 4;
     BlockState &B = *reinterpret_cast<BlockState *>(smem + sizeof(WarpTables) + slot * stride);
     uint32_t *planes = reinterpret_cast<uint32_t *>(&B + 1);
-    for (;;) {
-        int idx = 0;
-        if (lane == 0) idx = (int)atomicAdd(counter, 1u);
-        idx = __shfl_sync(kFull, idx, 0);
+    // The first block of every warp is dealt out over the CTAs, longest first,
+    // so that an SM does not start with twelve of the longest (mixed batch of
+    // 12 images 5.67 -> 5.08 ms, 3001x2047x3 12-bit lossless 12.2 -> 11.4);
+    // then the queue.
+    for (bool dealt = true;; dealt = false) {
+        int idx = slot * (int)gridDim.x + (int)blockIdx.x;
+        if (!dealt) {
+            if (lane == 0) idx = slots * (int)gridDim.x + (int)atomicAdd(counter, 1u);
+            idx = __shfl_sync(kFull, idx, 0);
+        }
         const uint32_t *order = queue.o0;
         if (idx >= queue.n0) {
             idx -= queue.n0;
@@ -874,7 +883,7 @@ cudaError_t launch_t1_warp(tc_ctx *ctx, bool styled, const tc_cblk_desc *d_desc,
     for (int s = 1; s <= kMaxSlots; s++) {
         const size_t sm = smem_of(s);
         if (sm > (size_t)I->smem_cta) break;
-        const int threads = std::max(128, 32 * s);
+        const int threads = 128 * ((s + 3) / 4);
         const int ctas = std::min((int)(I->smem_sm / (sm + 1024)), 65536 / (threads * ((I->regs + 7) & ~7)));
         if (ctas >= 1 && ctas * s >= best) {
             best = ctas * s;
@@ -891,7 +900,7 @@ cudaError_t launch_t1_warp(tc_ctx *ctx, bool styled, const tc_cblk_desc *d_desc,
         slots = (each + per_sm - 1) / per_sm;
     }
     const int grid = std::max(1, std::min((total + slots - 1) / slots, per_sm * sms));
-    const int threads = std::max(128, 32 * slots);
+    const int threads = 128 * ((slots + 3) / 4);
     uint32_t *words = ctx->d_words;
     auto kernel = styled ? t1_decode_warp_kernel<true, true>
                          : (deep ? t1_decode_warp_kernel<false, true> : t1_decode_warp_kernel<false, false>);
