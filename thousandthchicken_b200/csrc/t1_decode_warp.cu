@@ -400,7 +400,7 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
 #pragma unroll
             for (int half = 0; half < 2; half++) {
                 const int c = lane + 32 * half;
-                if (32 * half >= w) break;
+                if (32 * half >= w || (Raw && raw && type == 2)) break;
                 uint32_t l4;
                 if (type == 2) {
                     // 16 after the first refinement, else 15 with a
@@ -441,6 +441,21 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
             uint32_t vis = 0;   // lane j: the samples of word j coded in this pass
             if (type == 2) {
                 // ---- magnitude refinement (ISO D.3.3) ----
+                if (Raw && raw) {
+                    // raw bits, one a sample in scan order: no labels, no
+                    // contexts (1536x1100x3 lossless with bypass 4.27 -> 3.71 ms)
+                    do {
+                        const int j = __ffs(wm) - 1;
+                        wm &= wm - 1;
+                        uint32_t e = __shfl_sync(kFull, E, j), bits = 0;
+                        while (e) {
+                            const uint32_t bit = 1u << top_bit(e);
+                            e ^= bit;
+                            if (rw.bit()) bits |= bit;
+                        }
+                        if (lane == j) N = bits;
+                    } while (wm);
+                } else {
                 do {
                     const int j = __ffs(wm) - 1;
                     wm &= wm - 1;
@@ -496,6 +511,7 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
                     }
                     if (lane == j) N = bits;
                 } while (wm);
+                }
                 if (lane < 8) {
                     B.R[s * 8 + lane] |= E;
                     planes[p * kPlaneWords + s * 8 + lane] |= N;
