@@ -1,7 +1,8 @@
-// t1_common.cuh -- pieces shared by the Tier-1 decoder (t1_decode.cu) and
-// encoder (t1_encode.cu): the flag-word layout of a code-block's state, the
-// MQ probability-state table and the context-label tables (ISO Annex C.2,
-// D.3).  Included inside namespace tc's anonymous namespace of each file.
+// t1_common.cuh -- pieces shared by the Tier-1 decoders (t1_decode_warp.cu,
+// t1_decode.cu) and encoder (t1_encode.cu): the MQ probability-state table and
+// the zero-coding labels (ISO Annex C.2, D.3), the code-block style's passes,
+// and the flag-word layout and tables of t1_decode.cu.  Each file gets its own
+// copy in an anonymous namespace.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -14,7 +15,6 @@ namespace tc {
 namespace {
 
 constexpr int kMaxStripes = 16;    // 64 rows
-constexpr int kSgnCols = 66;       // 64 columns + a zero column on each side
 
 // Flag word layout (one per stripe column):
 //   bits 0-17  significance, bit 3*j + col for row j-1 of the stripe
@@ -44,7 +44,6 @@ __constant__ uint8_t c_nlps[47] = {
     38, 39, 40, 41, 42, 43, 46};
 
 struct Tables {
-    uint32_t mq[48];          // packed states: Qe << 16 | NMPS << 1 | NLPS << 7 | SWITCH << 13 (bit 0: MPS)
     uint8_t zc[4][512];       // zero-coding label per orientation and 3x3 neighbourhood
     uint8_t sc[256];          // sign label | XOR bit << 4
     // Decoder context words by 2 * state + MPS: Qe << 16, the entry after an
@@ -74,9 +73,6 @@ __device__ int zc_label(int orient, int h, int v, int d)
 
 __device__ void build_tables(Tables &t)
 {
-    for (int i = threadIdx.x; i < 47; i += blockDim.x)
-        t.mq[i] = ((uint32_t)c_qe[i] << 16) | ((uint32_t)c_nmps[i] << 1) | ((uint32_t)c_nlps[i] << 7) |
-                  ((uint32_t)(i == 0 || i == 6 || i == 14) << 13);
     for (int i = threadIdx.x; i < 94; i += blockDim.x) {
         const int st = i >> 1, mps = i & 1, sw = st == 0 || st == 6 || st == 14;
         t.mqd[i] = ((uint32_t)c_qe[st] << 16) | ((uint32_t)(2 * c_nlps[st] + (mps ^ sw)) << 7) |
@@ -110,45 +106,6 @@ __device__ void build_tables(Tables &t)
         }
         t.sc[i] = (uint8_t)(cx | (xr << 4));
     }
-}
-
-// Sign-coding index of row y (= 4s+k) of column c from the flag word's
-// 3x3 neighbourhood n9 and the sign words of columns c-1, c, c+1 (sgn has a
-// zero guard column on each side: column c is sgn[c + 1]).
-__device__ __forceinline__ uint32_t sign_index(const unsigned long long *sgn, uint32_t n9, int c, int y)
-{
-    const unsigned long long sl = sgn[c], sc = sgn[c + 1], sr = sgn[c + 2];
-    const uint32_t up = y > 0 ? (uint32_t)(sc >> (y - 1)) & 1u : 0u;
-    const uint32_t dn = y < 63 ? (uint32_t)(sc >> (y + 1)) & 1u : 0u;
-    const uint32_t lf = (uint32_t)(sl >> y) & 1u, rt = (uint32_t)(sr >> y) & 1u;
-    return (n9 & 0xAAu) | up | (lf << 2) | (rt << 4) | (dn << 6);
-}
-
-// Record that row k of stripe s in column c became significant: the flag
-// words of the neighbouring columns and of the stripes above and below see
-// it through their neighbourhood bits.  With vertically causal contexts
-// (vsc, ISO D.7) the stripe above does not: its last row's neighbourhood
-// then leaves out the row below for every context (zero coding, sign, run
-// mode, refinement).
-__device__ __forceinline__ void mark_significant(uint32_t *F, unsigned long long *sgn, int s, int k, int c, int w,
-                                                 int nstripes, uint32_t neg, bool vsc = false)
-{
-    const int i = s * 64 + c;
-    if (c > 0) F[i - 1] |= 1u << (3 * k + 5);
-    if (c + 1 < w) F[i + 1] |= 1u << (3 * k + 3);
-    if (k == 0 && s > 0 && !vsc) {
-        const int u = i - 64;
-        F[u] |= 1u << 16;
-        if (c > 0) F[u - 1] |= 1u << 17;
-        if (c + 1 < w) F[u + 1] |= 1u << 15;
-    }
-    if (k == 3 && s + 1 < nstripes) {
-        const int d = i + 64;
-        F[d] |= 1u << 1;
-        if (c > 0) F[d - 1] |= 1u << 2;
-        if (c + 1 < w) F[d + 1] |= 1u << 0;
-    }
-    if (neg) sgn[c + 1] |= 1ull << (4 * s + k);
 }
 
 // Code-block style (ISO Table A.19): whether coding pass t (0: the first
