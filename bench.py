@@ -960,7 +960,7 @@ def run_ours(args, rank, world, local_rank):
                                                                                     int(0.99 * len(srt)))], 3)},
             "stages_ms": {"tier1_dequant": round(t1_avg, 3), "dwt_colour": round(dwt_avg, 3)},
             "code_blocks_per_s": round(ncblk / (t1_avg / 1000.0), 1),
-            "roofline": {"bound": "issue", "kernel": "t1_decode_kernel",
+            "roofline": {"bound": "issue", "kernel": "t1_decode_warp_kernel",
                          "achieved": round(issue_achieved, 1) if issue_achieved else None,
                          "peak": round(issue_peak, 1), "unit": "G warp-instructions/s",
                          "frac": round(issue_achieved / issue_peak, 4) if issue_achieved else None,

@@ -4,9 +4,8 @@ Two choices are tuned, each on the plan's own work with CUDA events on its
 stream (tc_plan_stage_ms):
 
   * the Tier-1 lane-group width: 32 lanes per code-block (one warp per
-    block, eight per CTA), 16 (two blocks per warp) or 8 (four per warp,
-    decoded in lock-step); uniform blocks keep the groups of a warp in step,
-    ragged ones make them diverge;
+    block, a decoder of its own), 16 (two blocks per warp) or 8 (four per
+    warp, decoded in lock-step);
   * the staging of the fused last reverse 9/7 level: 2-D tensor copies (TMA)
     into persistent CTAs, or one 4-byte asynchronous copy per sample into a
     CTA per tile; large levels favour the first, small ones can favour the
