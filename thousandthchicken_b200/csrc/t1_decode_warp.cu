@@ -26,7 +26,7 @@
 // per block too), Tier-1 of one 64x64 block of 8 bit-planes 6.39 -> 3.06 ms,
 // of 14 bit-planes 10.4 -> 4.6 ms; 4096x4096x3 lossy 14.4 -> 13.3 ms (issue
 // 74% -> 80% of cycles, ALU pipe 74% busy), 2048x2048x3 12-bit lossless
-// 15.3 -> 8.7 ms.
+// 16.4 -> 8.7 ms.
 //
 // Code-blocks with a coding style (bypass, context reset, termination on every
 // pass, vertically causal contexts, segmentation symbols; ISO D.4-D.7) run in
