@@ -13,8 +13,8 @@
 //     significant makes five lanes recompute the labels that it changes, and a
 //     table lookup adds the samples that it makes candidates.  A run-length
 //     column is its first row alone, under its own label.
-//   * the serial part runs in lock-step on all lanes (uniform values, shared
-//     memory broadcasts); the next label and context word are loaded while the
+//   * the serial part runs on all lanes alike (see BlockState for what keeps
+//     them apart from one another's context words); the next label and context word are loaded while the
 //     current decision is decoded, and both successor states as soon as its
 //     context word is known.
 //   * magnitudes are bit-planes in shared memory (512 B each), gathered by the
@@ -45,6 +45,7 @@ namespace {
 constexpr int kRow = 9;          // words per stripe of a sample bitmap: 64 columns and a zero guard
 constexpr int kLabRun = 72, kLabUni = 68;   // context labels are kept as byte offsets (4 x label)
 constexpr int kMaxSlots = 12;    // code-blocks per CTA at most
+constexpr int kStyledSlots = 8;  // the same for styled blocks, which take up to 128 registers
 // Launches of fewer blocks per SM than this decode Deep: the label of the
 // sample after the next is loaded too and one branch leaves the straight line,
 // more instructions but shorter waits.  Against the other kernel: 1024x1024x3
@@ -61,19 +62,47 @@ struct WarpTables {
     uint2 adds[2][32];    // by pass (propagation, cleanup) and place: see build_warp_tables
 };
 
+// A context word: Qe << 16 | (2 x state + MPS) << 3.
+__device__ __forceinline__ uint32_t ctx_word(int state, int mps)
+{
+    return ((uint32_t)c_qe[state] << 16) | (uint32_t)((2 * state + mps) << 3);
+}
+
 // A code-block's state.  Bitmaps of samples have eight words a stripe, each
 // of eight columns of four rows, in scan order from the top bit down (column
 // c, row k: bit 31 - 4 (c & 7) - k, so that bit & 3 is 3 - k); a zero word
 // ends every stripe, and S and G have a zero stripe above and below.  The
 // magnitude bits follow as bit-planes of kPlaneWords words.
+//
+// All lanes run the serial part, but nothing keeps them in step there: a lane
+// must not store a context word that another has yet to read.  Deep: each lane
+// has context words of its own (21 words apart, so in different banks), and
+// between two new samples no lane waits for another.  Otherwise all share one
+// set, which keeps the state small, and a warp barrier stands before every
+// store; own sets, or contexts in registers and shuffles, cost such launches
+// more (4096x4096x3 lossy 13.6 ms with the barrier, 14.1 with sets for eight
+// lanes and 15.0 with shuffles; 2048x2048 16-bit lossless, Deep, 5.4 ms with
+// own words and 5.5 with the barrier).
+template <bool Deep>
 struct BlockState {
+    static constexpr int kSets = Deep ? 32 : 1;
+    static constexpr int kSetWords = Deep ? 21 : 20;
     uint32_t S[1 + 18 * kRow];   // significance (from S + 1: the guard before the first word)
     uint32_t G[1 + 18 * kRow];   // signs of the significant samples
     uint32_t P[16 * 8];          // coded in this plane's significance propagation pass
     uint32_t R[16 * 8];          // refined at least once
     uint32_t F[66];              // flag words of the current stripe's columns
     uint8_t lab[9 * 32];         // context label of every sample of the current stripe, in scan order
-    uint32_t ctx[20];            // context words
+    uint32_t ctx[kSets * kSetWords];   // context words
+
+    // The contexts' first states (ISO Table D.7).
+    __device__ void reset_contexts(int lane)
+    {
+        for (int i = lane; i < kSets * 19; i += 32) {
+            const int k = i / kSets;
+            ctx[i % kSets * kSetWords + k] = ctx_word(k == 0 ? 4 : (k == 17 ? 46 : (k == 18 ? 3 : 0)), 0);
+        }
+    }
 };
 constexpr int kPlaneWords = 128;
 
@@ -83,12 +112,6 @@ constexpr int kPlaneWords = 128;
 // columns to the left and to the right.  The 3x3 neighbourhood of row k is
 // (F >> 3 (3 - k)) & 0x1FF.
 constexpr int kOwnSign = 18, kLeftSign = 24, kRightSign = 28;
-
-// A context word: Qe << 16 | (2 x state + MPS) << 3.
-__device__ __forceinline__ uint32_t ctx_word(int state, int mps)
-{
-    return ((uint32_t)c_qe[state] << 16) | (uint32_t)((2 * state + mps) << 3);
-}
 
 __device__ void build_warp_tables(WarpTables &t)
 {
@@ -283,13 +306,13 @@ struct WarpRaw {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// Decode one code-block, all lanes in lock-step.  Returns the last pass type
+// Decode one code-block, all lanes alike.  Returns the last pass type
 // (0 cleanup, 1 significance propagation, 2 refinement) and its plane.
 // Modes: the code-block style `style` applies; lens, when not null, holds the
 // lengths of the codeword's terminated segments (BYPASS / TERMALL), which
 // follow one another from seg.  Raw: the block has raw (bypass) passes.
 template <bool Modes, bool Raw, bool Deep>
-__device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTables &T, const uint8_t *seg, int len, int w,
+__device__ int decode_block_warp(BlockState<Deep> &B, uint32_t *planes, const WarpTables &T, const uint8_t *seg, int len, int w,
                                  int h, int orient, int numbps, int passes, int *last_plane, int lane, int style,
                                  const uint32_t *lens)
 {
@@ -300,7 +323,7 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
     uint32_t segoff = 0;   // its first byte
     const bool vsc = Modes && (style & TC_CBLK_STYLE_VSC);
     if (!Modes || !lens) mq.init(seg, len);
-    char *ctxb = reinterpret_cast<char *>(B.ctx);
+    char *ctxb = reinterpret_cast<char *>(B.ctx + (Deep ? lane * B.kSetWords : 0));
     auto ctx_at = [&](int lab) -> uint32_t & { return *reinterpret_cast<uint32_t *>(ctxb + lab); };
     const uint8_t *zc = T.zc[orient];
     const int nstripes = (h + 3) >> 2;
@@ -316,6 +339,11 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
     // order: bit (at & lab_col) - lab_next.
     const int lab_col = lane < 4 ? ~3 : ~0, lab_next = lane < 4 ? lane + 1 : 1;
 
+    // Before a context word is stored that all lanes share.  No lane is then
+    // more than a decision ahead, which the labels and flag words need as well.
+    auto before_store = [&]() {
+        if constexpr (!Deep) __syncwarp();
+    };
     auto begin_pass = [&](int t) {
         if constexpr (Modes) {
             if (!lens || (t > 0 && !style_pass_terminates(style, t - 1))) return;
@@ -348,6 +376,7 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
     auto decide_now = [&](int lab) -> bool {
         uint32_t out;
         const bool d = mq.decide(T, ctx_at(lab), out);
+        before_store();
         ctx_at(lab) = out;
         return d;
     };
@@ -502,6 +531,7 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
                             uint32_t nx;
                             bool due;
                             if (decide(cw, nx, due)) bits |= bit;
+                            before_store();
                             ctx_at(lab) = nx;
                             if (!e) break;
                             cw = ln == lab ? nx : cn;
@@ -557,6 +587,7 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
                     uint32_t nx;
                     bool due;
                     const bool d = decide(cw, nx, due);
+                    before_store();
                     if (due) ctx_at(lab) = nx;
                     cw = due && ln == lab ? nx : cn;
                     // Deep: one branch leaves the straight line
@@ -581,7 +612,7 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
                             const int to = (at & lab_col) - lab_next;
                             uint32_t *fw = reinterpret_cast<uint32_t *>(fp - (to & ~3));
                             const bool other = ((to ^ at) & ~3) != 0;   // the next column
-                            __syncwarp();
+                            if constexpr (Deep) __syncwarp();   // else: the barrier before the store above
                             const uint32_t f = *reinterpret_cast<const uint32_t *>(fp - (at & ~3));
                             uint32_t v = *fw | ((other ? 32u : 16u) << (3 * r));
                             const uint2 add = adds[at];
@@ -603,6 +634,7 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
                             uint32_t snx;
                             bool sdue;
                             const bool neg = decide(sw, snx, sdue) != ((Raw && raw) ? false : (sv >> 7) != 0u);
+                            before_store();
                             if (sdue) ctx_at(sl) = snx;
                             if (neg) {
                                 v |= (other ? 1u << kLeftSign : 2u << kOwnSign) << r;
@@ -646,7 +678,7 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
             }
             if (style & TC_CBLK_STYLE_RESET) {
                 __syncwarp();
-                if (lane < 19) B.ctx[lane] = ctx_word(lane == 0 ? 4 : (lane == 17 ? 46 : (lane == 18 ? 3 : 0)), 0);
+                B.reset_contexts(lane);
             }
         }
         if (++t >= passes) break;
@@ -664,7 +696,7 @@ __device__ int decode_block_warp(BlockState &B, uint32_t *planes, const WarpTabl
 // Decode code-block `bi` with the state B and write it out.  np: the
 // bit-planes that the state has room for.
 template <bool Modes, bool Deep>
-__device__ __forceinline__ void process_block_warp(BlockState &B, uint32_t *planes, int np, const WarpTables &T,
+__device__ __forceinline__ void process_block_warp(BlockState<Deep> &B, uint32_t *planes, int np, const WarpTables &T,
                                                    const tc_cblk_desc *__restrict__ desc, uint32_t bi, int ndesc,
                                                    const uint8_t *__restrict__ pool, uint64_t pool_len,
                                                    char *__restrict__ out, uint64_t out_elems, int out_mode, float recon_r,
@@ -729,7 +761,7 @@ __device__ __forceinline__ void process_block_warp(BlockState &B, uint32_t *plan
     for (int i = lane; i < 1 + (nstripes + 2) * kRow; i += 32) B.S[i] = B.G[i] = 0u;
     for (int i = lane; i < nstripes * 8; i += 32) B.P[i] = B.R[i] = 0u;
     for (int i = lane; i < 9 * 8; i += 32) reinterpret_cast<uint32_t *>(B.lab)[i] = 0u;
-    if (lane < 19) B.ctx[lane] = ctx_word(lane == 0 ? 4 : (lane == 17 ? 46 : (lane == 18 ? 3 : 0)), 0);
+    B.reset_contexts(lane);
     __syncwarp();
 
     int type = 0, last_plane = 0;
@@ -805,7 +837,7 @@ struct BlockQueue {
 };
 
 template <bool Modes, bool Deep>
-__global__ void __launch_bounds__(32 * kMaxSlots, Modes ? 1 : 2)
+__global__ void __launch_bounds__(32 * (Modes ? kStyledSlots : kMaxSlots), 2)
 t1_decode_warp_kernel(const tc_cblk_desc *__restrict__ desc, BlockQueue queue, int ndesc, int slots, int np,
                       const uint8_t *__restrict__ pool, uint64_t pool_len, char *__restrict__ out, uint64_t out_elems,
                       int out_mode, float recon_r, uint32_t *__restrict__ counter, uint32_t *__restrict__ err)
@@ -818,8 +850,8 @@ t1_decode_warp_kernel(const tc_cblk_desc *__restrict__ desc, BlockQueue queue, i
     // the first (longest) blocks share theirs with the shortest or with none.
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = (warp & 4) ? warp ^ 3 : warp;
     if (slot >= slots) return;
-    const size_t stride = sizeof(BlockState) + (size_t)np * kPlaneWords * 4;
-    BlockState &B = *reinterpret_cast<BlockState *>(smem + sizeof(WarpTables) + slot * stride);
+    const size_t stride = sizeof(BlockState<Deep>) + (size_t)np * kPlaneWords * 4;
+    BlockState<Deep> &B = *reinterpret_cast<BlockState<Deep> *>(smem + sizeof(WarpTables) + slot * stride);
     uint32_t *planes = reinterpret_cast<uint32_t *>(&B + 1);
     // The first block of every warp is dealt out over the CTAs, longest first,
     // so that an SM does not start with twelve of the longest (mixed batch of
@@ -847,7 +879,8 @@ t1_decode_warp_kernel(const tc_cblk_desc *__restrict__ desc, BlockQueue queue, i
     }
 }
 
-static_assert(sizeof(WarpTables) % 16 == 0 && sizeof(BlockState) % 16 == 0, "state alignment");
+static_assert(sizeof(WarpTables) % 16 == 0 && sizeof(BlockState<false>) % 16 == 0 && sizeof(BlockState<true>) % 16 == 0,
+              "state alignment");
 
 struct WarpLaunch {
     int regs = 0;
@@ -892,11 +925,12 @@ cudaError_t launch_t1_warp(tc_ctx *ctx, bool styled, const tc_cblk_desc *d_desc,
                            : (deep ? warp_launch_info<false, true>(ctx, &I) : warp_launch_info<false, false>(ctx, &I));
     if (e != cudaSuccess) return e;
     const BlockQueue q{order[0], order[1], order[2], n[0], n[1], n[2]};
-    const size_t stride = sizeof(BlockState) + (size_t)max_planes * kPlaneWords * 4;
+    const size_t state = styled || deep ? sizeof(BlockState<true>) : sizeof(BlockState<false>);
+    const size_t stride = state + (size_t)max_planes * kPlaneWords * 4;
     auto smem_of = [&](int slots) { return sizeof(WarpTables) + slots * stride; };
     // CTA shape: the most code-blocks resident on an SM (24 for 8 bit-planes)
     int slots = 1, per_sm = 1, best = 0;
-    for (int s = 1; s <= kMaxSlots; s++) {
+    for (int s = 1; s <= (styled ? kStyledSlots : kMaxSlots); s++) {
         const size_t sm = smem_of(s);
         if (sm > (size_t)I->smem_cta) break;
         const int threads = 128 * ((s + 3) / 4);
