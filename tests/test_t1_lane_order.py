@@ -84,3 +84,16 @@ def test_warp_decoder_styles(emulated, style, order):
     _, desc, pool = codec.parse(codec.encode(img, 8, cblk_style=style, **kw))
     got = _decode(_warp(emulated, "styled", 12, order), desc, pool, want.size)
     np.testing.assert_array_equal(got.reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("order", ORDERS)
+@pytest.mark.parametrize("planes", [1, 6, 12])
+@pytest.mark.parametrize("lanes", [8, 16])
+def test_group_decoder(emulated, lanes, planes, order):
+    """Several blocks per warp: the groups' lanes part from one another, too."""
+    desc, pool = _blocks(planes)
+
+    def call(*a):
+        return emulated("EMU_GROUPS").emu_decode_groups(lanes, int(planes > 8), *a[:-1], order, a[-1])
+    got = _decode(call, desc, pool, len(desc) * SLOT)
+    np.testing.assert_array_equal(got.reshape(-1, 64, 64), oracle_slots(desc, pool, "int", 0.0))

@@ -17,7 +17,7 @@
 //     (sigma') bits of its four rows, and the signs of its six rows (-1..4).
 //     (The reference rebuilds a 3x3 window of packed words from global memory
 //     at every step, coefficient_coder.cl:271-298.)
-//   * a group's lanes run the decoder in lock-step; at every stripe they find
+//   * a group's lanes run the decoder alike; at every stripe they find
 //     the candidate columns of the pass with __ballot_sync and the serial loop
 //     visits only those;
 //   * the pass loop honours the coding-pass count (defect D3 fixed) and
@@ -112,6 +112,7 @@ struct MQ {
     const uint8_t *p;
     int len, bp, ct;
     uint32_t a, c, cur, nxt;
+    unsigned group;   // the lanes that decode this block
 
     __device__ __forceinline__ uint32_t byte_at(int i) const { return i < len ? (uint32_t)__ldg(p + i) : 0xFFu; }
     __device__ __forceinline__ void bytein()
@@ -132,10 +133,11 @@ struct MQ {
         cur = nxt;
         nxt = byte_at(bp + 1);   // used about nine decisions later: no prefetch needed
     }
-    __device__ __forceinline__ void init(const uint8_t *d, int n)
+    __device__ __forceinline__ void init(const uint8_t *d, int n, unsigned lanes)
     {
         p = d;
         len = n;
+        group = lanes;
         bp = 0;
         cur = byte_at(0);
         nxt = byte_at(1);
@@ -161,10 +163,13 @@ struct MQ {
     // One decision.  The interval arithmetic of ISO C.3.2 (both the MPS and
     // the LPS sub-interval, with the conditional exchange) is done with
     // selects; the one branch left is the renormalisation, which is also
-    // where the context's state moves on.
+    // where the context's state moves on.  The barrier keeps the group's lanes
+    // within a decision of one another: none stores a context or a flag word
+    // that another has yet to read as it was.
     __device__ __forceinline__ uint32_t decode(uint32_t *ctx, const uint32_t *tbl, int cx)
     {
         const uint32_t w = ctx[cx];
+        __syncwarp(group);
         const uint32_t qs = w & 0xFFFF0000u, mps = w & 1u;
         const uint32_t a1 = a - qs;
         const bool lower = c < qs;   // the code value lies in the Qe sub-interval
@@ -180,9 +185,9 @@ struct MQ {
     }
 };
 
-// Decode one code-block.  Every lane of the warp runs this function in
-// lock-step; lanes split the per-stripe candidate searches between them
-// (lane l owns columns l and l+32) and the serial loop visits only candidate
+// Decode one code-block.  Every lane of the group runs this function alike;
+// the lanes split the per-stripe candidate searches between them (lane l owns
+// columns l, l + G, ...) and the serial loop visits only candidate
 // columns, in scan order.  Returns the last pass type (0 cleanup,
 // 1 significance propagation, 2 refinement) and its plane.
 template <typename MagT, int G>
@@ -209,7 +214,7 @@ __device__ int decode_block(WarpState<MagT> &S, const Tables &T, const uint8_t *
         }
     };
     MQ mq;
-    mq.init(seg, len);
+    mq.init(seg, len, gmask);
     uint32_t *ctx = S.ctx;
     const uint32_t *tbl = T.mqd;
     const uint8_t *zc = T.zc[orient];
