@@ -1,8 +1,8 @@
 """The Tier-1 kernels' results do not depend on how far a lane runs ahead of
 the others between two synchronisation points (CUDA promises no lock-step
 there): the device code, run on the CPU warp emulator with its lanes taken in
-several orders, gives the oracle's samples, and every lane reaches the same
-synchronisation points."""
+several orders, gives the oracle's samples and the host encoder's codewords,
+and every lane reaches the same synchronisation points."""
 import ctypes as C
 
 import numpy as np
@@ -97,3 +97,25 @@ def test_group_decoder(emulated, lanes, planes, order):
         return emulated("EMU_GROUPS").emu_decode_groups(lanes, int(planes > 8), *a[:-1], order, a[-1])
     got = _decode(call, desc, pool, len(desc) * SLOT)
     np.testing.assert_array_equal(got.reshape(-1, 64, 64), oracle_slots(desc, pool, "int", 0.0))
+
+
+@pytest.mark.parametrize("order", ORDERS)
+@pytest.mark.parametrize("planes", [1, 6, 12])
+def test_encoder(emulated, planes, order):
+    rng = np.random.default_rng(planes)
+    cap = 8192
+    desc = np.zeros(4 * len(SIZES), codec.ENC_DESC_DTYPE)   # a CTA of four warps for each block
+    coefs = np.zeros(len(SIZES) * SLOT, np.int32)
+    want = []
+    for i, (w, h) in enumerate(SIZES):
+        coef = laplacian_block(rng, w, h, planes, zero_frac=0.3)
+        limit = int(rng.integers(1, 3 * planes - 1)) if i % 2 else 0
+        desc[4 * i] = (i * SLOT, w, 1.0, w, h, i % 4, 31, 0, limit)
+        coefs[i * SLOT:i * SLOT + w * h] = coef.ravel()
+        want.append(codec.t1_encode_block(coef, i % 4, 31, limit))
+    out, res = np.zeros(len(desc) * cap, np.uint8), np.zeros(len(desc), codec.ENC_RESULT_DTYPE)
+    assert emulated("EMU_ENCODE").emu_encode(_p(desc), len(desc), _p(coefs), _p(out), C.c_uint32(cap), _p(res), order) == 0
+    for i, (seg, passes, zbp) in enumerate(want):
+        r = res[4 * i]
+        assert (r["status"], r["passes"], r["zero_bitplanes"]) == (0, passes, zbp)
+        assert out[4 * i * cap:4 * i * cap + int(r["len"])].tobytes() == seg

@@ -10,7 +10,7 @@
 // serial: for every stripe of a pass the lanes work out in parallel which
 // samples the pass codes, their contexts and signs, and put the decisions
 // (context label, bit) into a list in scan order; the warp then runs the list
-// through the MQ coder in lock-step.
+// through the MQ coder, all lanes alike.
 //   * a lane holds two columns of the block (c and c + 32) as 64-bit masks in
 //     registers: significance, signs, the plane's bits, visited, refined; its
 //     neighbours' rows come by shuffles;
@@ -200,7 +200,12 @@ __device__ void encode_block(EncState &S, const EncTables &T, MQEnc &mq, const t
     const int w = d.w, h = d.h, nstripes = (h + 3) >> 2;
     const uint8_t *zc = T.zc[d.orient];
     char *ctxb = reinterpret_cast<char *>(S.ctx);
-    auto ctx_at = [&](uint32_t sym) -> uint32_t & { return *reinterpret_cast<uint32_t *>(ctxb + (sym & 0x7Cu)); };
+    auto ctx_at = [&](uint32_t sym) -> uint32_t { return *reinterpret_cast<const uint32_t *>(ctxb + (sym & 0x7Cu)); };
+    // all lanes run the list; none stores a word that another has yet to read
+    auto store_ctx = [&](uint32_t sym, uint32_t word) {
+        __syncwarp();
+        *reinterpret_cast<uint32_t *>(ctxb + (sym & 0x7Cu)) = word;
+    };
     unsigned long long sig[2] = {0ull, 0ull}, pi[2] = {0ull, 0ull}, ref[2] = {0ull, 0ull}, bits[2] = {0ull, 0ull};
     // six rows, -1..4, of stripe s of a column
     auto window = [](unsigned long long m, int s) -> uint32_t {
@@ -218,7 +223,7 @@ __device__ void encode_block(EncState &S, const EncTables &T, MQEnc &mq, const t
             const uint32_t s1 = S.sym[i];   // one past the end for the last
             const uint32_t cn = ctx_at(s1);
             const uint32_t nx = mq.encode(T, cw, s0 & 1u);
-            ctx_at(s0) = nx;
+            store_ctx(s0, nx);
             if (i >= n) break;
             cw = ((s0 ^ s1) & 0x7Cu) ? cn : nx;
             s0 = s1;
