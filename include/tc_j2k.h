@@ -151,7 +151,8 @@ typedef struct tc_cblk_desc {
  * irreversible path adds it on the last decoded plane, the reversible path
  * only for truncated blocks; 0 = truncated value).  max_bitplanes bounds
  * Mb - zero_bitplanes over the blocks (0 = up to 31); it sizes the
- * magnitude storage, and a block above it is flagged as out of range.
+ * magnitude storage, and a block above it is flagged as out of range.  A
+ * block's output words may hold part of its magnitudes until it is done.
  * d_out holds out_elems 4-byte elements: a block whose last sample,
  * out_off + (h-1)*out_pitch + w - 1, is not below out_elems is skipped before
  * anything is written and reported by tc_ctx_synchronize (the reference

@@ -18,11 +18,11 @@ ORDERS = [0, 1, 2, 3]   # ascending, descending, two shuffles
 SIZES = [(16, 12), (9, 7), (33, 5), (1, 6), (64, 8)]
 
 
-def _blocks(planes):
+def _blocks(planes, sizes=SIZES):
     rng = np.random.default_rng(planes)
-    desc = np.zeros(len(SIZES), codec.DESC_DTYPE)
+    desc = np.zeros(len(sizes), codec.DESC_DTYPE)
     segs, off = [], 0
-    for i, (w, h) in enumerate(SIZES):
+    for i, (w, h) in enumerate(sizes):
         coef = laplacian_block(rng, w, h, planes, zero_frac=0.3)
         coef[h // 2, w // 2] = (1 << planes) - 1
         seg, passes, zbp = codec.t1_encode_block(coef, i % 4, 31)
@@ -58,9 +58,11 @@ def _decode(call, desc, pool, elems):
     return out
 
 
-def _warp(emulated, kernel, planes, order):
+def _warp(emulated, kernel, planes, order, room=None):
+    """room: the bit-planes that a block's state holds (default: all)."""
     def call(*a):
-        return emulated("EMU_WARP").emu_decode(int(kernel == "styled"), int(kernel == "deep"), *a[:-1], planes, order, a[-1])
+        return emulated("EMU_WARP").emu_decode(int(kernel == "styled"), int(kernel == "deep"), *a[:-1], room or planes,
+                                               planes, order, a[-1])
     return call
 
 
@@ -70,6 +72,16 @@ def _warp(emulated, kernel, planes, order):
 def test_warp_decoder(emulated, kernel, planes, order):
     desc, pool = _blocks(planes)
     got = _decode(_warp(emulated, kernel, planes, order), desc, pool, len(desc) * SLOT)
+    np.testing.assert_array_equal(got.reshape(-1, 64, 64), oracle_slots(desc, pool, "int", 0.0))
+
+
+@pytest.mark.parametrize("planes,room", [(9, 8), (12, 11), (16, 8), (23, 11), (31, 8)])
+@pytest.mark.parametrize("kernel", ["lean", "deep", "styled"])
+def test_warp_decoder_moves_planes_on(emulated, kernel, planes, room):
+    """Blocks of more bit-planes than their state has room for, whole and cut
+    after any number of them: the samples that the state alone would give."""
+    desc, pool = _blocks(planes, SIZES[:4])
+    got = _decode(_warp(emulated, kernel, planes, 2, room), desc, pool, len(desc) * SLOT)
     np.testing.assert_array_equal(got.reshape(-1, 64, 64), oracle_slots(desc, pool, "int", 0.0))
 
 

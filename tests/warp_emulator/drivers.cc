@@ -41,7 +41,7 @@ enum { kOk = 0, kStuck = 1, kOutOfBounds = 2 };
 #if defined(EMU_WARP)
 template <bool Modes, bool Deep>
 static int decode(const tc_cblk_desc *desc, int n, const uint8_t *pool, uint64_t pool_len, uint32_t *out, uint64_t elems,
-                  int mode, float r, int planes, uint32_t seed, uint32_t *err)
+                  int mode, float r, int planes, int limit, uint32_t seed, uint32_t *err)
 {
     using namespace tc;
     const Order order(seed);
@@ -52,18 +52,19 @@ static int decode(const tc_cblk_desc *desc, int n, const uint8_t *pool, uint64_t
         build_warp_tables(T);
         __syncthreads();
         for (int i = 0; i < n; i++)
-            process_block_warp<Modes, Deep>(B, reinterpret_cast<uint32_t *>(&B + 1), planes, T, desc, (uint32_t)i, n, pool,
+            process_block_warp<Modes, Deep>(B, reinterpret_cast<uint32_t *>(&B + 1), planes, limit, T, desc, (uint32_t)i, n, pool,
                                             pool_len, reinterpret_cast<char *>(out), elems, mode, r, err, lane);
     });
     return !tables.intact() || !state.intact() ? kOutOfBounds : (ok ? kOk : kStuck);
 }
 
 extern "C" int emu_decode(int modes, int deep, const tc_cblk_desc *desc, int n, const uint8_t *pool, uint64_t pool_len,
-                          uint32_t *out, uint64_t elems, int mode, float r, int planes, uint32_t seed, uint32_t *err)
+                          uint32_t *out, uint64_t elems, int mode, float r, int planes, int limit, uint32_t seed,
+                          uint32_t *err)
 {
-    if (modes) return decode<true, true>(desc, n, pool, pool_len, out, elems, mode, r, planes, seed, err);
-    if (deep) return decode<false, true>(desc, n, pool, pool_len, out, elems, mode, r, planes, seed, err);
-    return decode<false, false>(desc, n, pool, pool_len, out, elems, mode, r, planes, seed, err);
+    if (modes) return decode<true, true>(desc, n, pool, pool_len, out, elems, mode, r, planes, limit, seed, err);
+    if (deep) return decode<false, true>(desc, n, pool, pool_len, out, elems, mode, r, planes, limit, seed, err);
+    return decode<false, false>(desc, n, pool, pool_len, out, elems, mode, r, planes, limit, seed, err);
 }
 #elif defined(EMU_GROUPS)
 template <typename MagT, int G>

@@ -665,8 +665,9 @@ cudaError_t launch_t1_decode(tc_ctx *ctx, const tc_cblk_desc *d_desc, const uint
 // Classes: blocks of <= 8, <= 16 and <= 31 coded bit-planes, in that order in
 // d_order (each slice longest first), then styled blocks in the same three.
 // One warp per block takes the three classes in one launch, the deepest (the
-// longest chains) first, with state for the deepest block (planes, or the
-// class's bound), and the styled ones in a launch of their own before it.
+// longest chains) first, whose state has room for the deepest block (planes, or
+// the class's bound) or less, and the styled ones in a launch of their own
+// before it.
 // With lane groups the plain classes run as concurrent launches, the 32- and
 // 16-bit ones on side streams; an 8-bit class at most half the size of the
 // 16-bit class joins its launch (a wider state decodes any narrower block).

@@ -19,9 +19,10 @@
 //     context word is known.
 //   * magnitudes are bit-planes in shared memory (512 B each), gathered by the
 //     epilogue with the inverse quantiser (ISO E.1); with the significance,
-//     sign, visited and refined bitmaps a block of 8 bit-planes takes 7 KB,
-//     and state is sized by the launch's deepest block, so that blocks of any
-//     depth share one launch.
+//     sign, visited and refined bitmaps a block of 8 bit-planes takes 7 KB.
+//     Blocks of any depth share one launch: when room for its deepest block
+//     would cost the others their places, deep blocks move their bits on to
+//     their output words (see kFewPlanes).
 // Against the decoder of per-column flag words that was here before (one warp
 // per block too), Tier-1 of one 64x64 block of 8 bit-planes 6.39 -> 3.06 ms,
 // of 14 bit-planes 10.4 -> 4.6 ms; 4096x4096x3 lossy 14.4 -> 13.3 ms (issue
@@ -105,6 +106,15 @@ struct BlockState {
     }
 };
 constexpr int kPlaneWords = 128;
+// A launch that does not fit the GPU at once with room for all bit-planes of
+// its deepest block, and that would fit more blocks with room for this many, has
+// room for no more than these places allow (11 with 24 places per SM); a deeper
+// block moves its bits to its output words as it goes.  So one deep block, or a
+// caller's bound of 31, costs the others no places: 4096x4096x3 lossy, blocks of
+// 4 bit-planes, with one block of 12 of its own 14.2 -> 12.5 ms, with one of 20
+// 16.4 -> 12.5, under a bound of 31 16.4 -> 12.5; 2048x2048x3 16-bit lossless
+// 13.4 -> 12.0.  A launch that fits anyway moves nothing.
+constexpr int kFewPlanes = 8;
 
 // Flag word of a stripe column: bits 3j + i (j = 0..5: rows 4..-1, i = 0
 // right, 1 this, 2 left column) significance; bits 18..23 the signs of the
@@ -306,15 +316,48 @@ struct WarpRaw {
 
 constexpr unsigned kFull = 0xffffffffu;
 
+// The magnitude bits of column x in stripe s, from n bit-planes after those in m.
+__device__ __forceinline__ void gather_planes(uint32_t (&m)[4], const uint32_t *planes, int n, int s, int x)
+{
+    const uint32_t *word = planes + s * 8 + (x >> 3);
+    const int sh = 28 - 4 * (x & 7);
+    for (int q = 0; q < n; q++) {
+        const uint32_t b = word[q * kPlaneWords] >> sh;
+#pragma unroll
+        for (int k = 0; k < 4; k++) m[k] = 2 * m[k] + ((b >> (3 - k)) & 1u);
+    }
+}
+
+// A state without room for another bit-plane: the np planes that it holds move
+// to the block's output words (more: below those that moved before).  A lane has
+// the same columns as in the epilogue, so no lane reads what another wrote.  Not
+// inlined: a block moves planes three times at most, and the serial part keeps
+// its registers.
+__device__ __noinline__ void move_planes(const uint32_t *planes, int np, uint32_t *ob, uint32_t pitch, int w, int h,
+                                         bool more, int lane)
+{
+    for (int s = 0; 4 * s < h; s++)
+        for (int x = lane; x < w; x += 32) {
+            uint32_t m[4] = {0u, 0u, 0u, 0u};
+            gather_planes(m, planes, np, s, x);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (4 * s + k >= h) break;
+                uint32_t *o = ob + (uint64_t)(4 * s + k) * pitch + x;
+                *o = more ? (*o << np) | m[k] : m[k];
+            }
+        }
+}
+
 // Decode one code-block, all lanes alike.  Returns the last pass type
 // (0 cleanup, 1 significance propagation, 2 refinement) and its plane.
 // Modes: the code-block style `style` applies; lens, when not null, holds the
 // lengths of the codeword's terminated segments (BYPASS / TERMALL), which
 // follow one another from seg.  Raw: the block has raw (bypass) passes.
 template <bool Modes, bool Raw, bool Deep>
-__device__ int decode_block_warp(BlockState<Deep> &B, uint32_t *planes, const WarpTables &T, const uint8_t *seg, int len, int w,
-                                 int h, int orient, int numbps, int passes, int *last_plane, int lane, int style,
-                                 const uint32_t *lens)
+__device__ int decode_block_warp(BlockState<Deep> &B, uint32_t *planes, int np, const WarpTables &T, const uint8_t *seg,
+                                 int len, int w, int h, int orient, int numbps, int passes, int *last_plane, int lane, int style,
+                                 const uint32_t *lens, uint32_t *ob, uint32_t pitch)
 {
     WarpMQ mq;
     WarpRaw rw;
@@ -382,10 +425,19 @@ __device__ int decode_block_warp(BlockState<Deep> &B, uint32_t *planes, const Wa
     };
 
     int type = 0, p = numbps - 1;
+    uint32_t *plane = planes - kPlaneWords;   // the bits of plane p
     for (int t = 0;;) {
         begin_pass(t);
-        if (type == 1 || t == 0)   // a new plane
-            for (int i = lane; i < nstripes * 8; i += 32) planes[p * kPlaneWords + i] = 0u;
+        if (type == 1 || t == 0) {   // a new plane
+            plane += kPlaneWords;
+            if (plane == planes + np * kPlaneWords) {
+                __syncwarp();
+                move_planes(planes, np, ob, pitch, w, h, p + 1 + np < numbps, lane);
+                __syncwarp();
+                plane = planes;
+            }
+            for (int i = lane; i < nstripes * 8; i += 32) plane[i] = 0u;
+        }
 
         for (int s = 0; s < nstripes; s++) {
             const int rows = min(4, h - 4 * s);
@@ -544,7 +596,7 @@ __device__ int decode_block_warp(BlockState<Deep> &B, uint32_t *planes, const Wa
                 }
                 if (lane < 8) {
                     B.R[s * 8 + lane] |= E;
-                    planes[p * kPlaneWords + s * 8 + lane] |= N;
+                    plane[s * 8 + lane] |= N;
                 }
                 continue;
             }
@@ -667,7 +719,7 @@ __device__ int decode_block_warp(BlockState<Deep> &B, uint32_t *planes, const Wa
                 const int i = 1 + (s + 1) * kRow + lane;
                 B.S[i] = S0 | N;
                 B.G[i] |= gn;
-                planes[p * kPlaneWords + s * 8 + lane] |= N;
+                plane[s * 8 + lane] |= N;
                 if (type == 1) B.P[s * 8 + lane] = vis;
             }
         }
@@ -694,9 +746,9 @@ __device__ int decode_block_warp(BlockState<Deep> &B, uint32_t *planes, const Wa
 }
 
 // Decode code-block `bi` with the state B and write it out.  np: the
-// bit-planes that the state has room for.
+// bit-planes that the state has room for; limit: the most that a block may have.
 template <bool Modes, bool Deep>
-__device__ __forceinline__ void process_block_warp(BlockState<Deep> &B, uint32_t *planes, int np, const WarpTables &T,
+__device__ __forceinline__ void process_block_warp(BlockState<Deep> &B, uint32_t *planes, int np, int limit, const WarpTables &T,
                                                    const tc_cblk_desc *__restrict__ desc, uint32_t bi, int ndesc,
                                                    const uint8_t *__restrict__ pool, uint64_t pool_len,
                                                    char *__restrict__ out, uint64_t out_elems, int out_mode, float recon_r,
@@ -711,7 +763,7 @@ __device__ __forceinline__ void process_block_warp(BlockState<Deep> &B, uint32_t
     const bool geom_ok = w >= 1 && w <= 64 && h >= 1 && h <= 64;
     const int numbps = (int)d.mb - (int)d.zero_bitplanes;
     bool ok = geom_ok && d.mb >= 1 && d.mb <= 31 && d.orient <= 3 && numbps >= 0 &&
-              (numbps == 0 || d.passes <= 3 * numbps - 2) && numbps <= np;
+              (numbps == 0 || d.passes <= 3 * numbps - 2) && numbps <= limit;
     const bool pool_ok = d.seg_off <= pool_len && (uint64_t)d.seg_len <= pool_len - d.seg_off;
     if (!geom_ok) {
         if (lane == 0) atomicOr(err, TC_DERR_DESC);
@@ -765,13 +817,14 @@ __device__ __forceinline__ void process_block_warp(BlockState<Deep> &B, uint32_t
     __syncwarp();
 
     int type = 0, last_plane = 0;
+    uint32_t *ob = reinterpret_cast<uint32_t *>(out) + d.out_off;   // the block's output words
     if (coded) {
         if (Modes && (style & TC_CBLK_STYLE_BYPASS) && d.passes > 10)
-            type = decode_block_warp<Modes, Modes, Deep>(B, planes, T, pool + cw_off, (int)d.seg_len, w, h, d.orient, numbps,
-                                                   d.passes, &last_plane, lane, style, lens);
+            type = decode_block_warp<Modes, Modes, Deep>(B, planes, np, T, pool + cw_off, (int)d.seg_len, w, h, d.orient,
+                                                          numbps, d.passes, &last_plane, lane, style, lens, ob, d.out_pitch);
         else
-            type = decode_block_warp<Modes, false, Deep>(B, planes, T, pool + cw_off, (int)d.seg_len, w, h, d.orient, numbps,
-                                                   d.passes, &last_plane, lane, style, lens);
+            type = decode_block_warp<Modes, false, Deep>(B, planes, np, T, pool + cw_off, (int)d.seg_len, w, h, d.orient,
+                                                          numbps, d.passes, &last_plane, lane, style, lens, ob, d.out_pitch);
     }
     __syncwarp();
 
@@ -781,6 +834,10 @@ __device__ __forceinline__ void process_block_warp(BlockState<Deep> &B, uint32_t
     const bool irrev = (d.flags & TC_CBLK_IRREVERSIBLE) != 0;
     const int roi = d.roi_shift < d.mb ? d.roi_shift : 0;
     const int mb_out = d.mb - roi;  // magnitude bits after the ROI shift
+    // the decoded bit-planes that are still in the state, after those that moved
+    const int nplanes = coded ? numbps - last_plane : 0;
+    int held = nplanes;
+    while (held > np) held -= np;
     for (int s = 0; s < nstripes; s++) {
         const int rows = min(4, h - 4 * s);
         for (int x = lane; x < w; x += 32) {
@@ -790,11 +847,12 @@ __device__ __forceinline__ void process_block_warp(BlockState<Deep> &B, uint32_t
                 sn = B.S[1 + (s + 1) * kRow + (x >> 3)] >> sh;
                 gn = B.G[1 + (s + 1) * kRow + (x >> 3)] >> sh;
                 pn = B.P[word] >> sh;
-                for (int q = numbps - 1; q >= last_plane; q--) {
-                    const uint32_t b = planes[q * kPlaneWords + word] >> sh;
+                if (nplanes > held) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) m[k] = 2 * m[k] + ((b >> (3 - k)) & 1u);
+                    for (int k = 0; k < 4; k++)
+                        if (k < rows) m[k] = ob[(uint64_t)(4 * s + k) * d.out_pitch + x];
                 }
+                gather_planes(m, planes, held, s, x);
             }
 #pragma unroll
             for (int k = 0; k < 4; k++) {
@@ -838,7 +896,7 @@ struct BlockQueue {
 
 template <bool Modes, bool Deep>
 __global__ void __launch_bounds__(32 * (Modes ? kStyledSlots : kMaxSlots), 2)
-t1_decode_warp_kernel(const tc_cblk_desc *__restrict__ desc, BlockQueue queue, int ndesc, int slots, int np,
+t1_decode_warp_kernel(const tc_cblk_desc *__restrict__ desc, BlockQueue queue, int ndesc, int slots, int np, int limit,
                       const uint8_t *__restrict__ pool, uint64_t pool_len, char *__restrict__ out, uint64_t out_elems,
                       int out_mode, float recon_r, uint32_t *__restrict__ counter, uint32_t *__restrict__ err)
 {
@@ -874,8 +932,8 @@ t1_decode_warp_kernel(const tc_cblk_desc *__restrict__ desc, BlockQueue queue, i
             }
         }
         const uint32_t bi = order ? order[idx] : (uint32_t)idx;
-        process_block_warp<Modes, Deep>(B, planes, np, T, desc, bi, ndesc, pool, pool_len, out, out_elems, out_mode, recon_r,
-                                  err, lane);
+        process_block_warp<Modes, Deep>(B, planes, np, limit, T, desc, bi, ndesc, pool, pool_len, out, out_elems, out_mode,
+                                        recon_r, err, lane);
     }
 }
 
@@ -926,26 +984,40 @@ cudaError_t launch_t1_warp(tc_ctx *ctx, bool styled, const tc_cblk_desc *d_desc,
     if (e != cudaSuccess) return e;
     const BlockQueue q{order[0], order[1], order[2], n[0], n[1], n[2]};
     const size_t state = styled || deep ? sizeof(BlockState<true>) : sizeof(BlockState<false>);
-    const size_t stride = state + (size_t)max_planes * kPlaneWords * 4;
-    auto smem_of = [&](int slots) { return sizeof(WarpTables) + slots * stride; };
-    // CTA shape: the most code-blocks resident on an SM (24 for 8 bit-planes)
-    int slots = 1, per_sm = 1, best = 0;
-    for (int s = 1; s <= (styled ? kStyledSlots : kMaxSlots); s++) {
-        const size_t sm = smem_of(s);
-        if (sm > (size_t)I->smem_cta) break;
-        const int threads = 128 * ((s + 3) / 4);
-        const int ctas = std::min((int)(I->smem_sm / (sm + 1024)), 65536 / (threads * ((I->regs + 7) & ~7)));
-        if (ctas >= 1 && ctas * s >= best) {
-            best = ctas * s;
-            slots = s;
-            per_sm = ctas;
+    const size_t plane = kPlaneWords * 4;
+    auto smem_of = [&](int slots, int np) { return sizeof(WarpTables) + slots * (state + np * plane); };
+    // CTA shape: the most code-blocks resident on an SM (24 for up to 8 bit-planes)
+    struct Shape {
+        int slots = 1, per_sm = 1, places = 0;
+    };
+    auto shape_of = [&](int np) {
+        Shape best;
+        for (int s = 1; s <= (styled ? kStyledSlots : kMaxSlots); s++) {
+            const size_t sm = smem_of(s, np);
+            if (sm > (size_t)I->smem_cta) break;
+            const int threads = 128 * ((s + 3) / 4);
+            const int ctas = std::min((int)(I->smem_sm / (sm + 1024)), 65536 / (threads * ((I->regs + 7) & ~7)));
+            if (ctas >= 1 && ctas * s >= best.places) best = Shape{s, ctas, ctas * s};
+        }
+        return best;
+    };
+    const int each = std::max(1, (total + sms - 1) / sms);
+    int np = max_planes;
+    Shape shape = shape_of(np);
+    if (np > kFewPlanes && shape.places < each) {
+        const Shape few = shape_of(kFewPlanes);
+        if (few.places > shape.places) {
+            shape = few;
+            while (smem_of(few.slots, np) > (size_t)I->smem_cta ||
+                   (int)(I->smem_sm / (smem_of(few.slots, np) + 1024)) < few.per_sm)
+                np--;
         }
     }
     // Blocks that all fit at once are spread evenly over the SMs: with 16 per
     // SM as two CTAs of 8 (1792x1792x3 lossy: 3.4 ms), not as 12 on every SM
     // and a second CTA on some of them (4.0 ms).
-    const int each = std::max(1, (total + sms - 1) / sms);
-    if (each < best) {
+    int slots = shape.slots, per_sm = shape.per_sm;
+    if (each < shape.places) {
         per_sm = (each + slots - 1) / slots;
         slots = (each + per_sm - 1) / per_sm;
     }
@@ -954,9 +1026,9 @@ cudaError_t launch_t1_warp(tc_ctx *ctx, bool styled, const tc_cblk_desc *d_desc,
     uint32_t *words = ctx->d_words;
     auto kernel = styled ? t1_decode_warp_kernel<true, true>
                          : (deep ? t1_decode_warp_kernel<false, true> : t1_decode_warp_kernel<false, false>);
-    kernel<<<grid, threads, smem_of(slots), ctx->stream>>>(d_desc, q, ndesc, slots, max_planes, d_pool, pool_len,
-                                                      static_cast<char *>(d_out), out_elems, out_mode, recon_r, words + word,
-                                                      words);
+    kernel<<<grid, threads, smem_of(slots, np), ctx->stream>>>(d_desc, q, ndesc, slots, np, max_planes, d_pool, pool_len,
+                                                               static_cast<char *>(d_out), out_elems, out_mode, recon_r,
+                                                               words + word, words);
     ctx->launches++;
     return cudaGetLastError();
 }

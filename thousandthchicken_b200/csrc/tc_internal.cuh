@@ -167,7 +167,7 @@ cudaError_t launch_t1_decode(tc_ctx *ctx, const tc_cblk_desc *d_desc, const uint
 // most 8, 16 and 31 coded bit-planes (n8 + n16 + n32 entries), then blocks
 // with a code-block style in the same three widths (nstyled[0..2], or none).
 // planes: the most coded bit-planes of a plain and of a styled block, when
-// the caller knows them (the decoder's state is sized for them).
+// the caller knows them (the decoder's state has room for no more).
 cudaError_t launch_t1_classes(tc_ctx *ctx, const tc_cblk_desc *d_desc, const uint32_t *d_order,
                               int ndesc, int n8, int n16, int n32, const uint8_t *d_pool,
                               uint64_t pool_len, void *d_out, uint64_t out_elems, int out_mode,
