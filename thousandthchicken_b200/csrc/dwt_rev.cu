@@ -361,10 +361,12 @@ __device__ __forceinline__ void rev_tile(const LevelIO &io, int bits, int bx, in
 
 // One level of one image: tiles (blockIdx.x, blockIdx.y), one component per
 // blockIdx.z for plane levels.
-// Four plane CTAs per SM (64 registers): without the bound 5/3 took more and
-// three, 2048x2048 in two waves (38 against 28 us); five spill (34 us).
+// Four CTAs of one-component tiles per SM (64 registers): without the bound 5/3
+// took more and three, 2048x2048 in two waves (38 against 28 us, and a grey
+// 2048x2048 image's last level 2 us longer); five spill (34 us).
 template <typename T, int WAVELET, int RND, int NCOMP, int COLOR, typename OT>
-__global__ void __launch_bounds__(kThreads, COLOR < 0 ? 4 : 1) idwt_rev_kernel(LevelIO io, int bits)
+__global__ void __launch_bounds__(kThreads, COLOR < 0 || NCOMP == 1 ? 4 : 1)
+    idwt_rev_kernel(LevelIO io, int bits)
 {
     pdl_allow_next();
     pdl_wait_prev();
@@ -376,8 +378,8 @@ __global__ void __launch_bounds__(kThreads, COLOR < 0 ? 4 : 1) idwt_rev_kernel(L
 // [jobs[j].tile0, jobs[j+1].tile0)), and each CTA finds its job by binary
 // search.
 template <typename T, int WAVELET, int RND, int NCOMP, int COLOR, typename OT>
-__global__ void __launch_bounds__(kThreads) idwt_rev_batch_kernel(const RevJob *__restrict__ jobs, int njobs,
-                                                                  int bits)
+__global__ void __launch_bounds__(kThreads, COLOR < 0 || NCOMP == 1 ? 4 : 1)
+    idwt_rev_batch_kernel(const RevJob *__restrict__ jobs, int njobs, int bits)
 {
     pdl_allow_next();
     const int b = blockIdx.x;
