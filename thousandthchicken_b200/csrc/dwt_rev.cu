@@ -131,8 +131,11 @@ __device__ __forceinline__ void rev_stage(const LevelIO &io, int bx, int by, int
         // two 8-byte stores) instead of four 4-byte copies, all loads in
         // flight at once.  Five reverse levels of 2048x2048: 9/7 35.1 -> 27.6
         // us, 5/3 34.8 -> 28.3; six of 4096x4096: 66.8 -> 62.4 and 68 -> 59 us.
+        // Not for several components: their copies are all in flight together,
+        // their loads into registers would follow one another (all levels of
+        // 2048x2048x4 5/3 75.6 against 86 us, 4096x4096x3 158 against 164).
         constexpr int SH = H % 4;   // columns of the first quad before the tile
-        const bool pairs = interior && x0 + TX + H + SH <= w && ((wl | io.ll_pitch | io.coef_pitch) & 1) == 0 &&
+        const bool pairs = NT == 1 && interior && x0 + TX + H + SH <= w && ((wl | io.ll_pitch | io.coef_pitch) & 1) == 0 &&
                            ((reinterpret_cast<uintptr_t>(ll) | reinterpret_cast<uintptr_t>(coef)) & 7) == 0;
         if (pairs) {
             using V2 = typename std::conditional<std::is_same<T, float>::value, float2, int2>::type;
