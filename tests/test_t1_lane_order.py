@@ -112,18 +112,22 @@ def test_group_decoder(emulated, lanes, planes, order):
 
 
 @pytest.mark.parametrize("order", ORDERS)
-@pytest.mark.parametrize("planes", [1, 6, 12])
-def test_encoder(emulated, planes, order):
+@pytest.mark.parametrize("planes", [0, 1, 6, 12])
+@pytest.mark.parametrize("irreversible", [False, True])
+def test_encoder(emulated, irreversible, planes, order):
+    """irreversible: float samples whose magnitudes are floored, zeros of either
+    sign among them; planes 0: empty blocks."""
     rng = np.random.default_rng(planes)
     cap = 8192
     desc = np.zeros(4 * len(SIZES), codec.ENC_DESC_DTYPE)   # a CTA of four warps for each block
-    coefs = np.zeros(len(SIZES) * SLOT, np.int32)
+    coefs = np.zeros(len(SIZES) * SLOT, np.float32 if irreversible else np.int32)
     want = []
     for i, (w, h) in enumerate(SIZES):
-        coef = laplacian_block(rng, w, h, planes, zero_frac=0.3)
-        limit = int(rng.integers(1, 3 * planes - 1)) if i % 2 else 0
-        desc[4 * i] = (i * SLOT, w, 1.0, w, h, i % 4, 31, 0, limit)
-        coefs[i * SLOT:i * SLOT + w * h] = coef.ravel()
+        coef = laplacian_block(rng, w, h, planes, zero_frac=0.3) if planes else np.zeros((h, w), np.int32)
+        limit = int(rng.integers(1, 3 * planes - 1)) if planes and i % 2 else 0
+        desc[4 * i] = (i * SLOT, w, 1.0, w, h, i % 4, 31, int(irreversible), limit)
+        fraction = np.where(coef == 0, rng.choice([-0.5, -0.0, 0.5], coef.shape), np.sign(coef) * 0.5) if irreversible else 0
+        coefs[i * SLOT:i * SLOT + w * h] = (coef + fraction).ravel()
         want.append(codec.t1_encode_block(coef, i % 4, 31, limit))
     out, res = np.zeros(len(desc) * cap, np.uint8), np.zeros(len(desc), codec.ENC_RESULT_DTYPE)
     assert emulated("EMU_ENCODE").emu_encode(_p(desc), len(desc), _p(coefs), _p(out), C.c_uint32(cap), _p(res), order) == 0

@@ -227,3 +227,4 @@ inline uint32_t __funnelshift_r(uint32_t lo, uint32_t hi, uint32_t s)
     return (uint32_t)(((uint64_t)hi << 32 | lo) >> (s & 31));
 }
 inline uint32_t __float_as_uint(float f) { return emu::value_of<uint32_t>(emu::bits_of(f)); }
+inline float __uint_as_float(uint32_t u) { return emu::value_of<float>(u); }

@@ -80,13 +80,16 @@ __device__ void build_enc_tables(EncTables &t)
     }
 }
 
-// Magnitude of sample (x, y) of block d: the int32 input, or the float input
-// quantised floor(|v| / step) (ISO E.2 deadzone).
-__device__ __forceinline__ uint32_t magnitude(const tc_t1_enc_desc &d, const void *in, int x, int y)
+// A sample's bits as they lie in the input, and their magnitude: the int32
+// input, or the float input quantised floor(|v| / step) (ISO E.2 deadzone).
+__device__ __forceinline__ uint32_t sample(const tc_t1_enc_desc &d, const void *in, int x, int y)
 {
-    const size_t i = d.in_off + (size_t)y * d.in_pitch + x;
-    if (d.flags & TC_CBLK_IRREVERSIBLE) return (uint32_t)floorf(fabsf(__ldg(static_cast<const float *>(in) + i)) * d.inv_step);
-    const int32_t v = __ldg(static_cast<const int32_t *>(in) + i);
+    return __ldg(static_cast<const uint32_t *>(in) + (d.in_off + (size_t)y * d.in_pitch + x));
+}
+__device__ __forceinline__ uint32_t magnitude(const tc_t1_enc_desc &d, uint32_t bits)
+{
+    if (d.flags & TC_CBLK_IRREVERSIBLE) return (uint32_t)floorf(fabsf(__uint_as_float(bits)) * d.inv_step);
+    const int32_t v = (int32_t)bits;
     return (uint32_t)(v < 0 ? -(int64_t)v : v);
 }
 
@@ -241,7 +244,7 @@ __device__ void encode_block(EncState &S, const EncTables &T, MQEnc &mq, const t
                 if (lane + 32 * j < w) {
 #pragma unroll 8
                     for (int y = 0; y < h; y++)
-                        m |= (unsigned long long)((magnitude(d, in, lane + 32 * j, y) >> p) & 1u) << y;
+                        m |= (unsigned long long)((magnitude(d, sample(d, in, lane + 32 * j, y)) >> p) & 1u) << y;
                 }
                 bits[j] = m;
                 pi[j] = 0ull;
@@ -381,21 +384,25 @@ __global__ void __launch_bounds__(32 * kEncWarps, 6)
         return;
     }
     // largest magnitude and the signs, rows coalesced across the lanes
-    const bool irrev = (d.flags & TC_CBLK_IRREVERSIBLE) != 0;
     uint32_t mx = 0;
     unsigned long long neg[2] = {0ull, 0ull};  // columns lane and lane + 32
-    for (int y = 0; y < h; y++) {
-        const size_t row = d.in_off + (size_t)y * d.in_pitch;
+    // Eight rows' loads in flight at once: a block with nothing to code is no more
+    // than this scan (12,000 empty 64x64 blocks, with the calls around the launch,
+    // 520 us row by row, 325 so; 3,000 of 9 bit-planes 6.74 -> 6.43 ms).
+    for (int y0 = 0; y0 < h; y0 += 8) {
+        uint32_t v[8][2];
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int x = lane + 32 * j;
-            if (x >= w) continue;
-            const uint32_t m = magnitude(d, in, x, y);
-            const bool ng = irrev ? static_cast<const float *>(in)[row + x] < 0.0f
-                                  : static_cast<const int32_t *>(in)[row + x] < 0;
-            mx = max(mx, m);
-            if (ng && m) neg[j] |= 1ull << y;
-        }
+        for (int k = 0; k < 8; k++)
+#pragma unroll
+            for (int j = 0; j < 2; j++) v[k][j] = y0 + k < h && lane + 32 * j < w ? sample(d, in, lane + 32 * j, y0 + k) : 0u;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const uint32_t m = magnitude(d, v[k][j]);
+                mx = max(mx, m);
+                if (m && (v[k][j] >> 31)) neg[j] |= 1ull << (y0 + k);
+            }
     }
     if (lane < 19) S.ctx[lane] = enc_word(lane == 0 ? 4 : (lane == 17 ? 46 : (lane == 18 ? 3 : 0)), 0);
     for (int i = lane; i < (int)sizeof S.sym; i += 32) S.sym[i] = 0;   // one past a list is read, too
