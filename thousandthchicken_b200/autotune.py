@@ -15,14 +15,17 @@ stream (tc_plan_stage_ms):
 The reference picks its DWT window by image width (DWTReverse53.cpp:36-42,
 DWTReverse97.cpp:37-43: 192, 128 or 64 columns); here the choice is
 measured.  `tune_plan` times the candidates, sets the winners on the plan's
-context and caches them in a JSON file keyed by GPU and bucket (image size
-class, code-block count class, image count class, wavelet mix, component
-count), so later plans of the same kind of batch skip the search.  Results
+context and caches them in a JSON file keyed by GPU, kernel revision and bucket
+(image size class, code-block count class, image count class, wavelet mix,
+component count), so later plans of the same kind of batch skip the search.  A
+choice timed with other kernels says nothing about these and is not applied.  Results
 do not depend on the choices (every candidate decodes bit for bit the
 same).
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import math
 import os
@@ -33,6 +36,20 @@ from . import _lib as L
 WIDTHS = (32, 16, 8)
 DWT_VARIANTS = {"tma": L.TC_DWT_TMA, "cp.async": L.TC_DWT_CPASYNC}
 CACHE = Path(os.environ.get("TC_J2K_TUNE_CACHE", Path(__file__).resolve().parent / "tune_cache.json"))
+
+
+@functools.lru_cache(maxsize=None)
+def revision() -> str:
+    """The kernels that choices were timed with: a hash of their sources."""
+    h = hashlib.sha256()
+    for f in sorted((Path(__file__).resolve().parent / "csrc").glob("*.cu*")):
+        h.update(f.name.encode() + b"\0" + f.read_bytes())
+    return h.hexdigest()[:16]
+
+
+def _prefix(ctx) -> str:
+    import torch
+    return f"{torch.cuda.get_device_name(ctx.device)}|{revision()}|"
 
 
 def _load():
@@ -72,10 +89,9 @@ def tune_plan(plan, outs, trials: int = 2, use_cache: bool = True) -> dict:
     """Pick the fastest Tier-1 lane-group width and last-level DWT staging
     for this plan's workload and set them on the plan's context.  Returns
     {"lanes", "dwt", "bucket", "tier1_ms", "dwt_ms", "cached"}."""
-    import torch
     ctx = plan.ctx
     b = bucket(plan)
-    key = f"{torch.cuda.get_device_name(ctx.device)}|{b}"
+    key = _prefix(ctx) + b
     cache = _load() if use_cache else {}
     if key in cache and "dwt" in cache[key]:
         c = cache[key]
@@ -121,12 +137,11 @@ def apply(plan, table: dict | None = None) -> dict | None:
     """Set the cached choices of the plan's bucket on its context (the
     defaults, TMA staging and 32 lanes, when the bucket was never tuned).
     `table` maps buckets to choices (default: the cache file)."""
-    import torch
     ctx = plan.ctx
     b = bucket(plan)
     if table is None:
-        table = {k.split("|", 1)[1]: v for k, v in _load().items()
-                 if k.startswith(torch.cuda.get_device_name(ctx.device) + "|")}
+        prefix = _prefix(ctx)
+        table = {k[len(prefix):]: v for k, v in _load().items() if k.startswith(prefix)}
     c = table.get(b)
     if c is None:
         _set(ctx, 32, L.TC_DWT_TMA)
