@@ -939,8 +939,8 @@ def run_ours(args, rank, world, local_rank):
         tf = ROOT / "profiles" / "ncu_traffic.json"
         if tf.exists():
             prof = json.loads(tf.read_text())
-        traffic = prof.get("t1_decode_kernel_bytes_per_launch")
-        inst = prof.get("t1_decode_kernel_inst_per_launch")
+        traffic = prof.get("t1_decode_warp_kernel_bytes_per_launch")
+        inst = prof.get("t1_decode_warp_kernel_inst_per_launch")
         if prof.get("inst_workload") != f"{W}x{H}x{Cn}":
             inst = None   # counted on another size
         # Tier-1 is bound by instruction issue: one warp instruction per

@@ -66,7 +66,7 @@ int tc_version(void);
 /* Number of kernel launches this ctx issued since creation (diagnostics). */
 uint64_t tc_ctx_launch_count(const tc_ctx *ctx);
 /* Lanes per code-block in the Tier-1 kernel: 32 (one warp per block), 16 or
- * 8 (two or four blocks per warp, decoded in lock-step).  The best width
+ * 8 (two or four blocks per warp).  The best width
  * depends on the block mix; the package's autotuner measures it per workload
  * and caches the choice.  Default 32. */
 int tc_ctx_set_t1_group(tc_ctx *ctx, int lanes);

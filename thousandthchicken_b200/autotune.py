@@ -5,7 +5,7 @@ stream (tc_plan_stage_ms):
 
   * the Tier-1 lane-group width: 32 lanes per code-block (one warp per
     block, a decoder of its own), 16 (two blocks per warp) or 8 (four per
-    warp, decoded in lock-step);
+    warp);
   * the staging of the fused last reverse 9/7 level: 2-D tensor copies (TMA)
     into persistent CTAs, or one 4-byte asynchronous copy per sample into a
     CTA per tile; large levels favour the first, small ones can favour the

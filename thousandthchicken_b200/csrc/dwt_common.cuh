@@ -48,10 +48,12 @@ __device__ __forceinline__ int pse(int i, int n)
 }
 
 // Index inside [0, n) after extension.  One reflection, without a division,
-// covers every signal longer than the halo; shorter ones take the general
-// form.  (With the general form alone, the border tiles that small levels
-// consist of spent most of their time on its division: reverse 9/7 of 512x512,
-// five levels, 35 against 27 us.)
+// covers the halo of every signal longer than it.  Signals shorter than the halo
+// take the general form, and so does the part of a tile that lies more than one
+// reflection past the end of a short level (samples that nobody stores).  (With
+// the general form alone, the border tiles that small levels consist of spent
+// most of their time on its division: reverse 9/7 of 512x512, five levels, 35
+// against 27 us.)
 __device__ __forceinline__ int mirror(int i, int n)
 {
     if ((unsigned)i < (unsigned)n) return i;

@@ -103,8 +103,8 @@ __device__ __forceinline__ int to_int(T v)
 template <typename T>
 using Vec4 = typename std::conditional<std::is_same<T, float>::value, float4, int4>::type;
 
-// Phase 1 of a tile: issues the asynchronous copies of tile (bx, by) of
-// level `io`, NT components from cbase, into `tiles` (the caller waits).
+// Phase 1 of a tile: stages tile (bx, by) of level `io`, NT components from
+// cbase, into `tiles` (the caller waits for the asynchronous copies among them).
 template <typename T, int WAVELET, int NT>
 __device__ __forceinline__ void rev_stage(const LevelIO &io, int bx, int by, int cbase, T *tiles)
 {
@@ -114,9 +114,10 @@ __device__ __forceinline__ void rev_stage(const LevelIO &io, int bx, int by, int
     const int x0 = bx * TX, y0 = by * TY;
     const int w = io.w, h = io.h, wl = (w + 1) >> 1, hl = (h + 1) >> 1;
 
-    // 1. load the extended tiles from the four subbands (Mallat layout) with
-    //    4-byte asynchronous copies, so a thread has its whole share of the
-    //    tile in flight at once.  x0 - H is even, so the parity of a column
+    // 1. load the extended tiles from the four subbands (Mallat layout), a
+    //    thread's whole share of the tile in flight at once: aligned interior
+    //    tiles of one component with 8-byte loads, the others with 4-byte
+    //    asynchronous copies.  x0 - H is even, so the parity of a column
     //    is the parity of the lane: inside the plane a lane's sources in a
     //    row are one strided run of the low or the high band.
     const bool interior = x0 >= H && x0 + TX + H <= w && y0 >= H && y0 + NR - H <= h;

@@ -398,7 +398,7 @@ __device__ int decode_block(WarpState<MagT> &S, const Tables &T, const uint8_t *
 }
 
 // Lanes per code-block G (16 or 8): a warp splits into 32 / G groups that
-// decode different code-blocks in lock-step (each group runs the serial
+// decode different code-blocks (each group runs the serial
 // decoder redundantly across its lanes and splits the candidate searches
 // between them), so one warp instruction can advance several code-blocks.
 // Code-blocks per CTA: the per-CTA label tables are shared by more blocks
@@ -410,7 +410,7 @@ struct GroupCfg {
 };
 
 // Decode code-block `bi` with the state S and write it out (the group's
-// lanes, in lock-step).  MagT bounds the coded bit-planes it accepts.
+// lanes, all alike).  MagT bounds the coded bit-planes it accepts.
 template <typename MagT, int G>
 __device__ __forceinline__ void process_block(WarpState<MagT> &S, const Tables &T, const tc_cblk_desc *__restrict__ desc,
                                               uint32_t bi, int ndesc, const uint8_t *__restrict__ pool,

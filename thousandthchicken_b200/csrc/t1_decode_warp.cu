@@ -24,10 +24,10 @@
 //     would cost the others their places, deep blocks move their bits on to
 //     their output words (see kFewPlanes).
 // Against the decoder of per-column flag words that was here before (one warp
-// per block too), Tier-1 of one 64x64 block of 8 bit-planes 6.39 -> 3.06 ms,
-// of 14 bit-planes 10.4 -> 4.6 ms; 4096x4096x3 lossy 14.4 -> 13.3 ms (issue
-// 74% -> 80% of cycles, ALU pipe 74% busy), 2048x2048x3 12-bit lossless
-// 16.4 -> 8.7 ms.
+// per block too), Tier-1 of one 64x64 block of 8 bit-planes 6.39 -> 3.03 ms,
+// of 14 bit-planes 10.4 -> 4.7 ms; 4096x4096x3 lossy 14.4 -> 12.6 ms (issue
+// 74% -> 87% of cycles, ALU pipe 76% busy), 2048x2048x3 12-bit lossless
+// 16.4 -> 9.0 ms.
 //
 // Code-blocks with a coding style (bypass, context reset, termination on every
 // pass, vertically causal contexts, segmentation symbols; ISO D.4-D.7) run in
@@ -50,9 +50,12 @@ constexpr int kStyledSlots = 8;  // the same for styled blocks, which take up to
 // Launches of fewer blocks per SM than this decode Deep: the label of the
 // sample after the next is loaded too and one branch leaves the straight line,
 // more instructions but shorter waits.  Against the other kernel: 1024x1024x3
-// lossy (5 blocks per SM) 1.85 and 2.05 ms, 2048x2048 16-bit lossless (7) 5.1
-// and 5.7, 1920x1080x3 lossy (12) 2.3 and 2.4; 1792x1792x3 lossy (16) 3.4 and
-// 3.2, 4096x4096x3 13.9 and 13.3.
+// lossy (5 blocks per SM) 1.86 and 2.12 ms, 2048x2048 16-bit lossless (7) 5.66
+// and 6.64; 1792x1792x3 lossy (16) 3.40 and 3.29, 4096x4096x3 13.8 and 12.6.
+// From 9 to 13 it depends on the blocks: where a few are much longer than the
+// rest Deep is faster (1472x1472x3 8-bit lossless 3.49 and 3.84, sparse lossy
+// 0.39 and 0.47), where all are alike the other one is (lossy 2.56 and 2.51,
+// 1536x1536x3 2.76 and 2.42).
 constexpr int kDeepBlocks = 13;
 
 // Label and probability tables of a CTA.
@@ -81,9 +84,9 @@ __device__ __forceinline__ uint32_t ctx_word(int state, int mps)
 // between two new samples no lane waits for another.  Otherwise all share one
 // set, which keeps the state small, and a warp barrier stands before every
 // store; own sets, or contexts in registers and shuffles, cost such launches
-// more (4096x4096x3 lossy 13.6 ms with the barrier, 14.1 with sets for eight
-// lanes and 15.0 with shuffles; 2048x2048 16-bit lossless, Deep, 5.4 ms with
-// own words and 5.5 with the barrier).
+// more (4096x4096x3 lossy 12.7 ms with the barrier, 13.9 with sets for eight
+// lanes; shuffles take 10% longer than the barrier.  2048x2048 16-bit lossless,
+// Deep, 5.2 ms with own words and 5.5 with the barrier).
 template <bool Deep>
 struct BlockState {
     static constexpr int kSets = Deep ? 32 : 1;
@@ -524,7 +527,7 @@ __device__ int decode_block_warp(BlockState<Deep> &B, uint32_t *planes, int np, 
                 // ---- magnitude refinement (ISO D.3.3) ----
                 if (Raw && raw) {
                     // raw bits, one a sample in scan order: no labels, no
-                    // contexts (1536x1100x3 lossless with bypass 4.27 -> 3.71 ms)
+                    // contexts (1536x1100x3 lossless with bypass: 3.77 ms, 0.55 less)
                     do {
                         const int j = __ffs(wm) - 1;
                         wm &= wm - 1;
@@ -913,7 +916,7 @@ t1_decode_warp_kernel(const tc_cblk_desc *__restrict__ desc, BlockQueue queue, i
     uint32_t *planes = reinterpret_cast<uint32_t *>(&B + 1);
     // The first block of every warp is dealt out over the CTAs, longest first,
     // so that an SM does not start with twelve of the longest (mixed batch of
-    // 12 images 5.67 -> 5.08 ms, 3001x2047x3 12-bit lossless 12.2 -> 11.4);
+    // 12 images 6.30 -> 5.49 ms, 3001x2047x3 12-bit lossless 12.98 -> 12.06);
     // then the queue.
     for (bool dealt = true;; dealt = false) {
         int idx = slot * (int)gridDim.x + (int)blockIdx.x;
@@ -1014,8 +1017,8 @@ cudaError_t launch_t1_warp(tc_ctx *ctx, bool styled, const tc_cblk_desc *d_desc,
         }
     }
     // Blocks that all fit at once are spread evenly over the SMs: with 16 per
-    // SM as two CTAs of 8 (1792x1792x3 lossy: 3.4 ms), not as 12 on every SM
-    // and a second CTA on some of them (4.0 ms).
+    // SM as two CTAs of 8 (1792x1792x3 lossy: 3.3 ms), not as 12 on every SM
+    // and a second CTA on some of them (0.6 ms more).
     int slots = shape.slots, per_sm = shape.per_sm;
     if (each < shape.places) {
         per_sm = (each + slots - 1) / slots;

@@ -22,7 +22,7 @@
 // The coder is bound by the decisions' chain when blocks are few and by issue
 // slots when they fill the GPU; the list takes the context search that ran
 // between decisions off both (64x64 blocks of 9 bit-planes: 48 of them 8.4 ->
-// 3.45 ms, 3,072 11.8 -> 7.6 ms, 12,288 42.2 -> 23.5 ms).  80 registers, six
+// 3.39 ms, 3,072 11.8 -> 7.4 ms, 12,288 42.2 -> 23.1 ms).  80 registers, six
 // CTAs (24 warps) per SM: at 96 and five, 768 CTAs left a second wave of 28
 // (8.1 ms); at 64 registers every block took 37% longer.
 #include <cuda_runtime.h>
