@@ -111,12 +111,13 @@ struct BlockState {
 constexpr int kPlaneWords = 128;
 // A launch that does not fit the GPU at once with room for all bit-planes of
 // its deepest block, and that would fit more blocks with room for this many, has
-// room for no more than these places allow (11 with 24 places per SM); a deeper
+// room for no more than these places allow (12 with 24 places per SM); a deeper
 // block moves its bits to its output words as it goes.  So one deep block, or a
-// caller's bound of 31, costs the others no places: 4096x4096x3 lossy, blocks of
-// 4 bit-planes, with one block of 12 of its own 14.2 -> 12.5 ms, with one of 20
-// 16.4 -> 12.5, under a bound of 31 16.4 -> 12.5; 2048x2048x3 16-bit lossless
-// 13.4 -> 12.0.  A launch that fits anyway moves nothing.
+// caller's bound of 31, costs the others no places: 4096x4096x3 lossy, most blocks
+// of 4 bit-planes, takes 12.6 ms alone, with one block of 20 and under a bound of
+// 31 (13.6, 16.4 and 16.4 before, with 24, 16 and 12 places; the first is the
+// code's difference), 2048x2048x3 16-bit lossless 12.0 (13.4).  A launch that fits
+// anyway moves nothing.
 constexpr int kFewPlanes = 8;
 
 // Flag word of a stripe column: bits 3j + i (j = 0..5: rows 4..-1, i = 0
